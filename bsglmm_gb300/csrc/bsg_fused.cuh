@@ -77,8 +77,19 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
   // other kernels keep one padded row per subject (a pad row per 32).
   constexpr bool PAIRX = !MIX && !SUPP;
   constexpr int RW = 2 * ((P + 1) & ~1);  // floats per pair row
-  constexpr int XS_FLOATS = PAIRX ? (kChunk / 2) * RW + (kChunk / 32) * 4 : kChunkPad * PP;
+  // subjects staged per pass: half a chunk for the t/logit links, whose two
+  // tables of Philox words would not fit 48 KB beside a whole one
+  constexpr int CH = MIX ? kChunk / 2 : kChunk;
+  constexpr int XS_FLOATS = PAIRX ? (CH / 2) * RW + (CH / 32) * 4 : (CH + CH / 32) * PP;
   __shared__ __align__(16) float Xs[XS_FLOATS];
+  // The words of the chunk's Philox calls that do not depend on the voxel
+  // (philox_q), one per call of four subjects (latent draws) and of two
+  // (t/logit weights); a pad entry per 32 subjects as for the design.  The
+  // heavy FMA pipe, which all products of the generator go through, is the
+  // busiest of the probit kernel (63 %): with a quarter of its products gone
+  // the sweep of N = 1000, P = 5 takes 0.517 ms instead of 0.531.
+  __shared__ uint4 Zq[SUPP ? 1 : CH / 4 + CH / 32];
+  __shared__ uint4 Pq[MIX ? CH / 2 + CH / 32 : 1];
   __shared__ float Om[P * P], Xtx[P * P];
 
   const BlockMap bm = map[blockIdx.x];
@@ -130,7 +141,11 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
   for (int q = 0; q < NQ; ++q) qw[q] = 0.f;
 
   PhiloxKey key;
-  if (!SUPP) key.init(ch.key0, ch.key1);
+  PhiloxLane vlane;
+  if (!SUPP) {
+    key.init(ch.key0, ch.key1);
+    vlane.init((uint32_t)v, sweep, key);
+  }
   int ok = 1;
   const uint32_t *yb = d.ybits[colour];
   // TC: the chunk's design slices and this warp's Z tile (dynamic shared
@@ -148,18 +163,29 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
     for (int q = 0; q < 4; ++q) tcd[jt][q] = 0.f;
   const bool run = TC ? __any_sync(0xffffffffu, active) : active;
 
-  for (int i0 = 0; i0 < N; i0 += kChunk) {
-    const int cn = min(kChunk, N - i0);
+  for (int i0 = 0; i0 < N; i0 += CH) {
+    const int cn = min(CH, N - i0);
+    const int cp = (cn + 31) & ~31;  // staged: whole words, x = 0 beyond N
     __syncthreads();
-    for (int t = tid; t < P * kChunk; t += blockDim.x) {
-      const int p = t / kChunk, ii = t - p * kChunk;
-      const float xv = ii < cn ? d.covar[(size_t)p * N + i0 + ii] : 0.f;
-      if constexpr (PAIRX) {
-        const int m = ii >> 1;
-        Xs[m * RW + (m >> 4) * 4 + 2 * p + (ii & 1)] = xv;
-      } else {
-        Xs[(ii + (ii >> 5)) * PP + p] = xv;
+    for (int ii = tid; ii < cp; ii += blockDim.x) {
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const float xv = ii < cn ? d.covar[(size_t)p * N + i0 + ii] : 0.f;
+        if constexpr (PAIRX) {
+          const int m = ii >> 1;
+          Xs[m * RW + (m >> 4) * 4 + 2 * p + (ii & 1)] = xv;
+        } else {
+          Xs[(ii + (ii >> 5)) * PP + p] = xv;
+        }
       }
+    }
+    if constexpr (!SUPP) {
+      for (int t = tid; t < cp / 4; t += blockDim.x)
+        Zq[t + (t >> 3)] = philox_q((uint32_t)((i0 >> 2) + t), sweep, cid | kTagZ, key);
+    }
+    if constexpr (MIX) {
+      for (int t = tid; t < cp / 2; t += blockDim.x)
+        Pq[t + (t >> 4)] = philox_q((uint32_t)((i0 >> 1) + t), sweep, cid | kTagPhi, key);
     }
     if constexpr (TC) tc_stage_design<P>(tc_smem, d.covar, N, i0, cn, tid, blockDim.x);
     __syncthreads();
@@ -170,12 +196,7 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
       auto subject = [&](int col, uint32_t ymask, uint32_t kk, uint32_t isub,
                          uint32_t gn, uint32_t gu, float ph) {
         float x[P];
-        if constexpr (PAIRX) {
-          const int ii = col - col / 33, m = ii >> 1;  // col = ii + ii / 32
-          const float *xr = &Xs[m * RW + (m >> 4) * 4 + (ii & 1)];
-#pragma unroll
-          for (int p = 0; p < P; ++p) x[p] = xr[2 * p];
-        } else {
+        {
           const float4 v0 = *reinterpret_cast<const float4 *>(&Xs[col * PP]);
           x[0] = v0.x;
           if (P > 1) x[1] = v0.y;
@@ -245,12 +266,7 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         }
         const float zr = m0 + __uint_as_float(__float_as_uint(t) ^ ymask ^ 0x80000000u);
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-          if constexpr (PAIRX)
-            acc2[p].x = fmaf(x[p], zr, acc2[p].x);
-          else
-            acc[p] = fmaf(x[p], zr, acc[p]);
-        }
+        for (int p = 0; p < P; ++p) acc[p] = fmaf(x[p], zr, acc[p]);
       };
       // The probit groups on subject pairs (PAIRX): G groups of four subjects
       // (G Philox calls), x'beta, the inversion and X'(Z - bwm) each as 2G
@@ -305,7 +321,7 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         if (__any_sync(__activemask(), amax > kATail)) {
 #pragma unroll
           for (int q = 0; q < 2 * H; ++q)
-            if (aq[q] > kATail) {
+            if (aq[q] > kATail && i + q < (uint32_t)N) {
               const uint32_t ym = (ywg >> q) << 31;
               const float t = tn_lower_tail(aq[q], i + q, (uint32_t)v, sweep,
                                             cid | kTagZTail, ch.key0, ch.key1, &ok);
@@ -451,90 +467,100 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         return pick4(r, q);
       };
       const int nw = (cn + 31) >> 5;
+      // The outcome word is loaded one word ahead: taken where it is used, its
+      // load stalled a warp 0.85 cycles per issue (0.49 now); sweep of N = 2000,
+      // P = 8 4 % shorter, of 1.5M voxels, N = 500 3.4 %.
+      auto yload = [&](int wl) -> uint32_t {
+        return (wl >= nw || (TC && !active)) ? 0u
+                                             : __ldg(yb + (size_t)((i0 >> 5) + wl) * nc + j);
+      };
+      uint32_t ynext = yload(k);
       for (int wl = k; wl < nw; wl += LPV) {
-        const int w = (i0 >> 5) + wl;
-        uint32_t yw = (TC && !active) ? 0u : __ldg(yb + (size_t)w * nc + j);
+        uint32_t yw = ynext;
+        ynext = yload(wl + LPV);
         const int nbits = min(32, cn - (wl << 5));
         const int xo = (wl << 5) + wl;  // padded offset of bit 0
         const uint32_t i00 = (uint32_t)(i0 + (wl << 5));
-        // MIX: the gamma variates of subjects i, i + 1 come from counter
-        // i / 2 (normal, uniform each)
-        auto gpair = [&](uint32_t i) -> uint4 {
-          if (!MIX) return make_uint4(0, 0, 0, 0);
-          return philox(make_uint4(i >> 1, (uint32_t)v, sweep, cid | kTagPhi), key);
+        // the latent words of subjects 4c..4c+3 of this word; MIX: the gamma
+        // variates of subjects 2c, 2c + 1 (normal, uniform each)
+        const uint4 *zq = &Zq[SUPP ? 0 : 9 * wl], *pq = &Pq[MIX ? 17 * wl : 0];
+        auto zcall = [&](int c) -> uint4 {
+          return SUPP ? make_uint4(0, 0, 0, 0) : philox_qv(zq[c], vlane, key);
+        };
+        auto gpair = [&](int c) -> uint4 {
+          return MIX ? philox_qv(pq[c], vlane, key) : make_uint4(0, 0, 0, 0);
         };
         // MIX: the weights phi of a group of four subjects are loaded one
         // group ahead (the stores of the current group may alias as far as
         // the compiler knows, so it would not hoist them itself)
         const float *phb = MIX ? ch.phi[colour] + j : nullptr;
-        // (TC: a ragged last word also takes the whole-word path; its
-        // subjects beyond the chunk have x = 0 and add nothing)
-        if (TC || nbits == 32) {
+        if constexpr (PAIRX) {
+          // whole steps of kGroups calls, then (the end of a ragged last
+          // word) steps of two calls or one; the subjects beyond N have
+          // x = 0 and add nothing (TC: the whole word)
+          const int nb = TC ? 32 : nbits;
+#pragma unroll 1
+          for (int b = 0; b < nb;) {
+            const uint32_t i = i00 + (uint32_t)b;
+            auto step = [&](auto gsz) {
+              constexpr int G = decltype(gsz)::value;
+              uint4 rs[G];
+#pragma unroll
+              for (int q = 0; q < G; ++q) rs[q] = zcall((b >> 2) + q);
+              groupp(gsz, (wl << 5) + b, yw, rs, i);
+              yw = G == 8 ? 0u : yw >> (4 * G);
+              b += 4 * G;
+            };
+            const int left = nb - b;
+            if (TC || left > 4 * (kGroups - 1)) {
+              step(std::integral_constant<int, kGroups>{});
+              if constexpr (TC) {
+                if ((b & 8) == 0) {  // a 16-subject slice is complete
+                  __syncwarp();
+                  tc_slice<P>(tc_smem, ((wl << 5) + b - 8) >> 4, tc_zt, tid & 31, tcd);
+                  __syncwarp();
+                }
+              }
+            } else if (kGroups > 2 && left > 4) {
+              step(std::integral_constant<int, 2>{});
+            } else {
+              step(std::integral_constant<int, 1>{});
+            }
+          }
+        } else if (nbits == 32) {
           float phc[4] = {1.f, 1.f, 1.f, 1.f}, phx[4] = {1.f, 1.f, 1.f, 1.f};
           if (MIX) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) phc[q] = phb[(size_t)(i00 + q) * nc];
           }
-          if constexpr (PAIRX) {
 #pragma unroll 1
-            for (int b = 0; b < 32; b += 4 * kGroups) {
-              const uint32_t i = i00 + (uint32_t)b;
-              uint4 rs[kGroups];
+          for (int b = 0; b < 32; b += 4) {
+            const uint32_t i = i00 + (uint32_t)b;
+            if (MIX && b + 4 < 32) {
 #pragma unroll
-              for (int q = 0; q < kGroups; ++q)
-                rs[q] = philox(make_uint4((i >> 2) + q, (uint32_t)v, sweep, cid | kTagZ), key);
-              groupp(std::integral_constant<int, kGroups>{}, (wl << 5) + b, yw, rs, i);
-              yw >>= 4 * kGroups;
-              if constexpr (TC) {
-                if (b & 8) {  // a 16-subject slice is complete
-                  __syncwarp();
-                  tc_slice<P>(tc_smem, ((wl << 5) + b) >> 4, tc_zt, tid & 31, tcd);
-                  __syncwarp();
-                }
+              for (int q = 0; q < 4; ++q) phx[q] = phb[(size_t)(i + 4 + q) * nc];
+            }
+            const uint4 r = zcall(b >> 2);
+            if constexpr (MIX) {
+              group4_mix(xo + b, yw, r, i, gpair(b >> 1), gpair((b >> 1) + 1), phc);
+              yw >>= 4;
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                subject(xo + b + q, yw << 31, variate(r, q, i + q), i + q, 0u, 0u, phc[q]);
+                yw >>= 1;
               }
             }
-          } else {
-#pragma unroll 1
-            for (int b = 0; b < 32; b += 4) {
-              const uint32_t i = i00 + (uint32_t)b;
-              if (MIX && b + 4 < 32) {
+            if (MIX) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) phx[q] = phb[(size_t)(i + 4 + q) * nc];
-              }
-              uint4 r = make_uint4(0, 0, 0, 0);
-              if (!SUPP) r = philox(make_uint4(i >> 2, (uint32_t)v, sweep, cid | kTagZ), key);
-              if constexpr (MIX) {
-                group4_mix(xo + b, yw, r, i, gpair(i), gpair(i + 2), phc);
-                yw >>= 4;
-              } else {
-                const uint4 g0 = gpair(i), g1 = gpair(i + 2);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const uint4 gq = q < 2 ? g0 : g1;
-                  subject(xo + b + q, yw << 31, variate(r, q, i + q), i + q,
-                          (q & 1) ? gq.z : gq.x, (q & 1) ? gq.w : gq.y, phc[q]);
-                  yw >>= 1;
-                }
-              }
-              if (MIX) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) phc[q] = phx[q];
-              }
+              for (int q = 0; q < 4; ++q) phc[q] = phx[q];
             }
           }
         } else {
           for (int b = 0; b < nbits; b += 4) {
             const uint32_t i = i00 + (uint32_t)b;
-            uint4 r = make_uint4(0, 0, 0, 0);
-            if (!SUPP) r = philox(make_uint4(i >> 2, (uint32_t)v, sweep, cid | kTagZ), key);
-            if constexpr (PAIRX) {
-              if (b + 4 <= nbits) {  // a whole group of the last word
-                groupp(std::integral_constant<int, 1>{}, (wl << 5) + b, yw, &r, i);
-                yw >>= 4;
-                continue;
-              }
-            }
-            const uint4 g0 = gpair(i), g1 = gpair(i + 2);
+            const uint4 r = zcall(b >> 2);
+            const uint4 g0 = gpair(b >> 1), g1 = gpair((b >> 1) + 1);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const uint4 gq = q < 2 ? g0 : g1;

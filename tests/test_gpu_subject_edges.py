@@ -1,0 +1,48 @@
+"""The colour kernels' subject loop at the sizes where its steps change: the
+ends of a ragged last outcome word (16-, 8- and 4-subject steps, the last one
+partly beyond N) and the edges of a staged pass (1024 subjects, 512 for the
+t/logit links), against the FP64 oracle chain on the same counters.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from bsglmm_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+# one sweep of FP32 draws from the oracle's (the bound of the other oracle
+# comparisons of single sweeps)
+TOL = 1e-4
+
+
+def _P(N):
+    """Covariates: one for the few-subject studies, whose isolated voxel would
+    otherwise have a singular X'X and no neighbour to add Omega."""
+    return 1 if N < 8 else 3 + N % 2
+
+
+@pytest.mark.parametrize("step", [8, 16])
+@pytest.mark.parametrize("N", [1, 3, 4, 5, 8, 9, 12, 13, 16, 17, 31, 33, 1023, 1024, 1029])
+def test_probit_sweep_matches_oracle(oracle_mod, N, step):
+    import bsglmm_gb300 as bsg
+    st = synth.small_study(300 + N, shape=(6, 5, 6), N=N, P=_P(N), S=1)
+    with bsg.Sampler() as s:
+        ch = s.add_chain(s.add_dataset(st.mask, st.covar, st.data, 1), seed=7)
+        s.set_step_subjects(step)
+        s.run(1)
+        o = oracle_mod.Problem(st.mask, st.covar, st.data, 1).chain(7, 1)
+        assert np.allclose(s.beta(ch), o["beta"], rtol=TOL, atol=TOL)
+
+
+@pytest.mark.parametrize("N", [1, 30, 32, 35, 511, 512, 513, 1030])
+def test_t_sweep_matches_oracle(oracle_mod, N):
+    import bsglmm_gb300 as bsg
+    st = synth.small_study(400 + N, shape=(6, 5, 6), N=N, P=_P(N), S=1)
+    with bsg.Sampler() as s:
+        ch = s.add_chain(s.add_dataset(st.mask, st.covar, st.data, 1), seed=9)
+        s.set_model(ch, "t")
+        s.run(1)
+        o = oracle_mod.Problem(st.mask, st.covar, st.data, 1).chain(9, 1, model=2)
+        assert np.allclose(s.beta(ch), o["beta"], rtol=TOL, atol=TOL)
