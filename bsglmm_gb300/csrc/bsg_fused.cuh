@@ -280,8 +280,12 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
       // (G = 2 gives four chains and was measured 1.6 % faster per sweep
       // than G = 1).  The results do not depend on G.
       constexpr int kGroups = WIDE ? 4 : 2;
-      auto groupp = [&](auto gsz, int ii0, uint32_t ywg, const uint4 *rs, uint32_t i) {
+      // A last group that reaches beyond N (`rag`) adds its one to three
+      // subjects in order to the even sums, those beyond N not at all.
+      auto groupp = [&](auto gsz, auto rag, int ii0, uint32_t ywg, const uint4 *rs,
+                        uint32_t i) {
         constexpr int G = decltype(gsz)::value;
+        [[maybe_unused]] constexpr bool RAG = decltype(rag)::value;
         constexpr int H = 2 * G;
         const int m = ii0 >> 1;  // a multiple of H: rows m..m+H-1 share one pad group
         const float *xr0 = &Xs[m * RW + (m >> 4) * 4];
@@ -341,6 +345,16 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
 #pragma unroll
             for (int h = 0; h < 4; ++h) zz[h] = active ? zh[h] : make_float2(0.f, 0.f);
             tc_store_z(tc_zt, tid & 31, (ii0 >> 3) & 1, zz);
+          }
+        } else if constexpr (RAG) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            const float *xr = xr0 + (q >> 1) * RW + (q & 1);
+            const float z = (q & 1) ? zh[q >> 1].y : zh[q >> 1].x;
+            if (i + q < (uint32_t)N) {
+#pragma unroll
+              for (int p = 0; p < P; ++p) acc2[p].x = fmaf(xr[2 * p], z, acc2[p].x);
+            }
           }
         } else {
 #pragma unroll
@@ -496,24 +510,24 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         const float *phb = MIX ? ch.phi[colour] + j : nullptr;
         if constexpr (PAIRX) {
           // whole steps of kGroups calls, then (the end of a ragged last
-          // word) steps of two calls or one; the subjects beyond N have
-          // x = 0 and add nothing (TC: the whole word)
+          // word) steps of two calls or one, the last one perhaps reaching
+          // beyond N (TC: the whole word, x = 0 beyond N)
           const int nb = TC ? 32 : nbits;
 #pragma unroll 1
           for (int b = 0; b < nb;) {
             const uint32_t i = i00 + (uint32_t)b;
-            auto step = [&](auto gsz) {
+            auto step = [&](auto gsz, auto rag) {
               constexpr int G = decltype(gsz)::value;
               uint4 rs[G];
 #pragma unroll
               for (int q = 0; q < G; ++q) rs[q] = zcall((b >> 2) + q);
-              groupp(gsz, (wl << 5) + b, yw, rs, i);
+              groupp(gsz, rag, (wl << 5) + b, yw, rs, i);
               yw = G == 8 ? 0u : yw >> (4 * G);
               b += 4 * G;
             };
             const int left = nb - b;
-            if (TC || left > 4 * (kGroups - 1)) {
-              step(std::integral_constant<int, kGroups>{});
+            if (TC || left >= 4 * kGroups) {
+              step(std::integral_constant<int, kGroups>{}, std::false_type{});
               if constexpr (TC) {
                 if ((b & 8) == 0) {  // a 16-subject slice is complete
                   __syncwarp();
@@ -521,10 +535,12 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
                   __syncwarp();
                 }
               }
-            } else if (kGroups > 2 && left > 4) {
-              step(std::integral_constant<int, 2>{});
+            } else if (kGroups > 2 && left >= 8) {
+              step(std::integral_constant<int, 2>{}, std::false_type{});
+            } else if (left >= 4) {
+              step(std::integral_constant<int, 1>{}, std::false_type{});
             } else {
-              step(std::integral_constant<int, 1>{});
+              step(std::integral_constant<int, 1>{}, std::true_type{});
             }
           }
         } else if (nbits == 32) {
