@@ -39,7 +39,7 @@ SOURCES = [
     "bsg_api.cpp",
 ]
 HEADERS = ["bsg_device.cuh", "bsg_fused.cuh", "bsg_internal.h", "bsg_math.cuh",
-           "bsg_wishart.cuh", "bsg_mma.cuh"]
+           "bsg_wishart.cuh", "bsg_mma.cuh", "bsg_mills_table.h"]
 
 
 def nvcc() -> str:

@@ -45,7 +45,8 @@ struct Group {
   int P = 0;
   bool mix = false;     // t/logit chains (scale-mixture colour kernel)
   bool wm_any = false;  // its chains draw beta_WM: colour 0 waits for it
-  bool fp64 = false;    // FP64 chains (fp64_colour_kernel, no early start)
+  int fp64 = 0;         // lanes per voxel of FP64 chains (fp64_colour_kernel,
+                        // no early start); 0: FP32
   bool wide = false;    // the 16-subject whole-word step (bsg_fused_wide.cu)
   double vox = 0, subj_vox = 0;  // its chains' voxels and N x voxels
   std::vector<BlockMap> map[2];
@@ -259,14 +260,26 @@ std::string status_text(int bits) {
 
 constexpr int kParityThreads = 128;  // tile of the supplied-variate sweep
 
+// Lanes per voxel of an FP64 chain: four while one lane each would put fewer
+// than eight warps on an SM of a GB300 (152 x 8 x 32 voxels of a colour), one
+// above, where four would only idle three lanes of each coefficient draw.
+// By the study alone, so that a chain's sums do not depend on what else its
+// context holds.  Measured at 9,424 voxels a colour, N = 117, P = 4: 0.79 ms
+// per sweep with one lane, 0.48 ms with four.
+int f64_lanes(const Dataset &d) {
+  return std::max(d.vox[0].size(), d.vox[1].size()) < 38912 ? kF64Lanes : 1;
+}
+
 // Partials of the colour kernels, one per block of a chain and value
 // (value-major, so that the last block's sums read consecutive blocks):
 // column sums (colour 0) and pairs + column sums (colour 1), sized for the
 // smallest tile the context launches; tot0 takes colour 0's totals.
 bsg_status ensure_partials(bsg_ctx *ctx, int vpb) {
   cudaError_t e;
+  const int vpb32 = vpb;
   for (auto &c : ctx->ch) {
     const Dataset &d = ctx->ds[c.dataset];
+    const int vpb = c.dev.fp64 ? std::min(vpb32, kF64Threads / f64_lanes(d)) : vpb32;
     const size_t n0 = std::max<size_t>(1, (d.vox[0].size() + vpb - 1) / vpb);
     const size_t n1 = std::max<size_t>(1, (d.vox[1].size() + vpb - 1) / vpb);
     if (n0 > c.cap0) {
@@ -327,7 +340,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
   const int vpb = ctx->threads / ctx->lpv;
   // partial rows for the smallest tile any kernel of this context uses
   bsg_status ps = ensure_partials(
-      ctx, std::min({vpb, kParityThreads, ctx->threads / kMixLpv, kF64Threads}));
+      ctx, std::min({vpb, kParityThreads, ctx->threads / kMixLpv}));
   if (ps) return ps;
   std::vector<DatasetDev> hds;
   for (auto &d : ctx->ds) hds.push_back(d.dev);
@@ -347,7 +360,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
     const Dataset &d = ctx->ds[ctx->ch[ci].dataset];
     const bool mix = ctx->ch[ci].dev.model != 1;
     const bool wmu = ctx->ch[ci].dev.wm_update != 0;
-    const bool f64 = ctx->ch[ci].dev.fp64 != 0;
+    const int f64 = ctx->ch[ci].dev.fp64 ? f64_lanes(d) : 0;
     Group *g = nullptr;
     for (auto &gg : ctx->groups)
       if (gg.P == d.P && gg.mix == mix && gg.wm_any == wmu && gg.fp64 == f64) g = &gg;
@@ -360,8 +373,8 @@ bsg_status build_plan(bsg_ctx *ctx) {
       g->fp64 = f64;
     }
     // the t/logit kernel runs kMixLpv lanes per voxel, the beta_WM one one,
-    // the FP64 one one thread per voxel in blocks of kF64Threads
-    const int gvpb = f64 ? kF64Threads
+    // the FP64 one f64 lanes per voxel in blocks of kF64Threads
+    const int gvpb = f64 ? kF64Threads / f64
                          : (mix ? ctx->threads / kMixLpv : (wmu ? ctx->threads : vpb));
     for (int c = 0; c < 2; ++c) map_chain(g->map[c], (int)ci, (int)d.vox[c].size(), gvpb, c);
     g->vox += (double)d.V;
@@ -429,7 +442,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
 // One colour kernel of a group.
 cudaError_t launch_colour(bsg_ctx *ctx, const Group &g, int c, cudaStream_t st, bool pdl) {
   if (g.fp64)
-    return launch_fp64(g.P, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
+    return launch_fp64(g.P, g.fp64, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
                        st);
   if (g.mix)
     return launch_fused_mix(g.P, ctx->threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
@@ -1130,7 +1143,7 @@ int64_t bsg_launches_per_sweep(const bsg_ctx *ctx) {
   for (auto &c : ctx->ch) {
     const Dataset &d = ctx->ds[c.dataset];
     const int P = d.P * 8 + (c.dev.model != 1) * 2 + (c.dev.wm_update != 0) +
-                  (c.dev.fp64 != 0) * 4;
+                  (c.dev.fp64 ? 4 + (f64_lanes(d) > 1) : 0);
     const int PS = d.P * 16 + d.S;
     if (std::find(ps.begin(), ps.end(), P) == ps.end()) ps.push_back(P);
     if (c.pred_on && std::find(pp.begin(), pp.end(), PS) == pp.end()) pp.push_back(PS);

@@ -6,25 +6,104 @@
 // covar.cpp:121-325 and mcmc.cpp:584-651 on the same counters), fast enough
 // to run the long reference chains that the FP32 sampler's maps are
 // measured against at the brain-sized studies, where the CPU would take
-// days.  It is written for agreement, not speed: one thread per voxel,
-// subjects in order, CUDA's double-precision normcdf / normcdfinv.
+// days.  One thread per voxel, subjects in order, or (studies with too few
+// voxels to fill the GPU) four lanes per voxel.
+//
+// What bounds it is the FP64 pipe (two lanes per clock and SM: a warp's
+// operation takes 16 cycles), so the latent draw is written for FP64
+// operations: about 63 + 2 P per subject and voxel.  CUDA's normcdf and
+// normcdfinv, which it used before, took some 330 and 2,120 instructions in
+// all, since the lanes of a warp go down both branches of each.
+#include "bsg_mills_table.h"
 #include "bsg_wishart.cuh"
 
 namespace bsg {
 namespace {
 
 constexpr int kF64Chunk = 512;  // subjects of the design staged per pass
+constexpr int kF64Unroll = 2;   // subjects drawn side by side
 
-// N(0,1) truncated to (a, +inf) by inversion of u(k), in FP64:
-// t = Phi^-1(Phi(a) + u Q(a)).  For a >= 0 the argument is at least 1/2 and
-// t = -Phi^-1(Q(a) (1 - u)); for a < 0 the small Phi(a) keeps its relative
-// precision and Q(a) = 1 - Phi(a) is at least 1/2.  1 - u = u(~k).
-__device__ double tn_lower_inv_d(double a, uint32_t k) {
-  const double uc = u_of_d(~k);
-  if (a >= 0.0) return -normcdfinv(normcdf(-a) * uc);
-  const double pa = normcdf(a), qa = 1.0 - pa;
-  const double pl = pa + u_of_d(k) * qa;
-  return pl < 0.5 ? normcdfinv(pl) : -normcdfinv(qa * uc);
+// The tables of the draw, in shared memory (lanes index them apart).
+struct DrawTables {
+  double mills[kMillsCoef][kMillsRows];
+  double exp2[64];
+};
+
+__device__ void load_tables(DrawTables &tb, int tid, int nthreads) {
+  for (int t = tid; t < kMillsRows * kMillsCoef; t += nthreads)
+    tb.mills[t % kMillsCoef][t / kMillsCoef] = kMillsTable[t];
+  for (int t = tid; t < 64; t += nthreads) tb.exp2[t] = kExp2Table[t];
+}
+
+// Mills ratio (1 - Phi(x)) / phi(x) for x >= 0: the row of the nearest
+// multiple of 1/8, found by adding 1.5 * 2^49 (whose last place is 1/8), and
+// a polynomial of degree 8 in the difference.  Beyond the table (x > 11.06)
+// the last row's centre: there Q(x) < 1e-28 only ever meets u >= 2^-33.
+__device__ __forceinline__ double mills(double x, const DrawTables &tb) {
+  const double m = x + 0x1.8p49;
+  const uint32_t j = (uint32_t)__double2loint(m);
+  double h = x - (m - 0x1.8p49);
+  if (j >= (uint32_t)kMillsRows) h = 0.0;
+  const uint32_t r = min(j, (uint32_t)kMillsRows - 1u);
+  double c = tb.mills[kMillsCoef - 1][r];
+#pragma unroll
+  for (int i = kMillsCoef - 2; i >= 0; --i) c = fma(c, h, tb.mills[i][r]);
+  return c;
+}
+
+// exp(y) for y <= 700 by a table of 2^(j/64) and a polynomial of degree 5
+// (Tang 1989); below -700 it stays at exp(-700).  n log(2)/64 is exact in its
+// leading part for the |n| < 2^17 that occur.
+__device__ __forceinline__ double exp_tab(double y, const DrawTables &tb) {
+  if ((uint32_t)__double2hiint(y) > 0xC085E000u) y = -700.0;
+  const double m = fma(y, 9.23324826168936568e+01, 0x1.8p52);
+  const int n = __double2loint(m);
+  const double k = m - 0x1.8p52;
+  const double r = fma(k, -2.98158582698529328e-12, fma(k, -0x1.62e42fee00000p-7, y));
+  double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+  q = fma(q, r, 1.0 / 6.0);
+  q = fma(q, r, 0.5);
+  q = fma(q, r, 1.0);
+  const double t = tb.exp2[n & 63];
+  const double e = fma(t, q * r, t);
+  return __hiloint2double(__double2hiint(e) + ((n >> 6) << 20), __double2loint(e));
+}
+
+__device__ __forceinline__ double flip_sign_d(double x, bool flip) {
+  return __hiloint2double(__double2hiint(x) ^ (flip ? (int)0x80000000 : 0), __double2loint(x));
+}
+
+// N(0,1) truncated to (a, +inf), a <= kATail, by inversion of u(k) in FP64:
+// t = Phi^-1(Phi(a) + u Q(a)).  With T = Q(|a|) the upper tail of t is
+// p = T (1 - u) for a >= 0 and (1 - u) - T (1 - u) for a < 0; there, where
+// the lower tail p = u + T (1 - u) is below 1/2, it is taken instead, so that
+// the small side keeps its relative precision.  x = Q^-1(p) starts from the
+// FP32 sampler's inversion (relative error d of 1e-6) and takes one step of
+// the series of Q(x + d) = p to third order, which leaves d^4:
+//   F = (Q(x) - p) / phi(x) = R(x) - p sqrt(2 pi) exp(x^2 / 2),
+//   d = F + x F^2 / 2 + (2 x^2 + 1) F^3 / 6.
+__device__ __forceinline__ double tn_lower_inv_d(double a, uint32_t k, const DrawTables &tb) {
+  constexpr double kSqrt2Pi = 2.50662827463100069;
+  // u = (k + 1/2) 2^-32 exactly, from the double 2^52 + k; so is 1 - u
+  const double u = fma(__hiloint2double(0x43300000, (int)k), 0x1p-32, -0x1p20 + 0x1p-33);
+  const double uc = 1.0 - u;
+  const bool neg = a < 0.0;
+  const double ax = fabs(a);
+  // FP32: which tail, and the starting point
+  const float fu = u_of(k), fuc = u_of(~k), fT = phi_tail((float)ax);
+  const float ftuc = __fmul_rn(fT, fuc), fq = fmaf(fT, fuc, fu);
+  const bool lo = neg && fq < 0.5f;
+  const float x0 = -ndtri_lower(lo ? fq : (neg ? __fsub_rn(fuc, ftuc) : ftuc));
+  // T sqrt(2 pi) = R(|a|) exp(-a^2 / 2), a^2 with its rounding error
+  const double a2 = ax * ax, a2l = fma(ax, ax, -a2);
+  const double T = mills(ax, tb) * (exp_tab(-0.5 * a2, tb) * fma(-0.5, a2l, 1.0));
+  const double A = lo ? u : (neg ? uc : 0.0);
+  const double p = fma(flip_sign_d(uc, neg && !lo), T, A * kSqrt2Pi);
+  const double x = (double)x0, xx = x * x;
+  const double F = fma(-p, exp_tab(0.5 * xx, tb), mills(x, tb));
+  double d = fma(F, fma(xx, 1.0 / 3.0, 1.0 / 6.0), 0.5 * x);
+  d = fma(F, d, 1.0);
+  return flip_sign_d(fma(F, d, x), lo);
 }
 
 // a > kATail: the Robert (1995) exponential-proposal rejection of
@@ -68,12 +147,17 @@ __device__ double sum_rows(const double *base, int nrow, int lane) {
   return s;
 }
 
-template <int P>
+// LPV lanes per voxel, each taking every LPV-th group of four subjects.  A
+// warp alone issues an FP64 operation every 80 cycles or so (18,848 voxels on
+// one lane each put two warps on an SM: FP64 pipe 38 % busy), and four or five
+// fill the pipe; see f64_lanes for the rule.
+template <int P, int LPV>
 __global__ void __launch_bounds__(kF64Threads)
     fp64_colour_kernel(const DatasetDev *__restrict__ dsv, ChainDev *__restrict__ chv,
                        const BlockMap *__restrict__ map, int colour) {
   constexpr int NT = P * (P + 1) / 2;
-  __shared__ float Xs[kF64Chunk * P];
+  __shared__ DrawTables tb;
+  __shared__ double Xs[kF64Chunk * P];
   __shared__ double Om[P * P], Xtx[P * P];
   __shared__ double red[kF64Threads / 32][kFusedVals];
   __shared__ double tot[kFusedVals];
@@ -84,7 +168,8 @@ __global__ void __launch_bounds__(kF64Threads)
   const DatasetDev &d = dsv[ch.dataset];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nc = d.n[colour];
-  const int j = bm.start + tid;
+  const int lane_v = tid % LPV;  // this lane's share of the subjects
+  const int j = bm.start + tid / LPV;
   const bool active = j < nc;
   const int N = d.N, Vp = d.Vp;
   const long long sweep_ll = ch.sweep[colour];
@@ -107,6 +192,7 @@ __global__ void __launch_bounds__(kF64Threads)
   }
   int ok = 1;
   const uint32_t *yb = d.ybits[colour];
+  load_tables(tb, tid, blockDim.x);
 
   // ---- latent Z_iv for every subject, accumulated into X'(Z - b_WM WM)
   // (updateZ, covar.cpp:302-325, and the b of Spat_Coefff, covar.cpp:142-150)
@@ -115,36 +201,61 @@ __global__ void __launch_bounds__(kF64Threads)
     __syncthreads();
     for (int t = tid; t < P * cn; t += blockDim.x) {
       const int p = t / cn, ii = t - p * cn;
-      Xs[ii * P + p] = d.covar[(size_t)p * N + i0 + ii];
+      Xs[ii * P + p] = (double)d.covar[(size_t)p * N + i0 + ii];
     }
     __syncthreads();
     if (!active) continue;
-    uint4 r = make_uint4(0, 0, 0, 0);
-    uint32_t yw = 0;
-    for (int ii = 0; ii < cn; ++ii) {
-      const int i = i0 + ii;  // i0 is a multiple of 32
-      if ((i & 31) == 0) yw = __ldg(yb + (size_t)(i >> 5) * nc + j);
-      if ((i & 3) == 0)
-        r = philox1(make_uint4((uint32_t)(i >> 2), (uint32_t)v, sweep, cid | kTagZ),
-                    ch.key0, ch.key1);
-      double x[P], mu = bwm;
+    auto yload = [&](int ii) -> uint32_t {
+      return ii < cn ? __ldg(yb + (size_t)((i0 + ii) >> 5) * nc + j) : 0u;
+    };
+    uint32_t ynext = yload(4 * lane_v);
+    for (int ii0 = 4 * lane_v; ii0 < cn; ii0 += 4 * LPV) {
+      const uint32_t yw = ynext;
+      ynext = yload(ii0 + 4 * LPV);
+      const uint4 r = philox1(make_uint4((uint32_t)((i0 + ii0) >> 2), (uint32_t)v, sweep,
+                                         cid | kTagZ), ch.key0, ch.key1);
+      // kF64Unroll subjects at a time (their draws are independent and hide
+      // each other's latency); the last group may be short
 #pragma unroll
-      for (int p = 0; p < P; ++p) {
-        x[p] = (double)Xs[ii * P + p];
-        mu += beta[p] * x[p];
+      for (int h = 0; h < 4; h += kF64Unroll) {
+        const int ii = ii0 + h, i = i0 + ii;  // i0 is a multiple of 32
+        if (ii >= cn) break;
+        double mu[kF64Unroll], t[kF64Unroll], a[kF64Unroll];
+        bool y[kF64Unroll];
+        bool far = false;
+#pragma unroll
+        for (int q = 0; q < kF64Unroll; ++q) {
+          const int iq = min(ii + q, cn - 1);  // (a short group repeats its last)
+          mu[q] = bwm;
+#pragma unroll
+          for (int p = 0; p < P; ++p) mu[q] += beta[p] * Xs[iq * P + p];
+          y[q] = (yw >> ((i + q) & 31)) & 1u;
+          a[q] = flip_sign_d(mu[q], y[q]);
+          t[q] = tn_lower_inv_d(a[q], pick4(r, h + q), tb);
+          far = far || a[q] > (double)kATail;
+        }
+        if (far) {
+#pragma unroll
+          for (int q = 0; q < kF64Unroll; ++q)
+            if (a[q] > (double)kATail && ii + q < cn)
+              t[q] = tn_lower_tail_d(a[q], (uint32_t)(i + q), (uint32_t)v, sweep,
+                                     cid | kTagZTail, ch.key0, ch.key1, &ok);
+        }
+#pragma unroll
+        for (int q = 0; q < kF64Unroll; ++q) {
+          if (ii + q < cn) {
+            const double zr = mu[q] + flip_sign_d(t[q], !y[q]) - bwm;  // Z - b_WM WM
+#pragma unroll
+            for (int p = 0; p < P; ++p) acc[p] += Xs[(ii + q) * P + p] * zr;
+          }
+        }
       }
-      const bool y = (yw >> (i & 31)) & 1u;
-      const double a = y ? -mu : mu;
-      const double t =
-          a <= (double)kATail
-              ? tn_lower_inv_d(a, pick4(r, i & 3))
-              : tn_lower_tail_d(a, (uint32_t)i, (uint32_t)v, sweep, cid | kTagZTail,
-                                ch.key0, ch.key1, &ok);
-      const double zr = mu + (y ? t : -t) - bwm;  // Z - b_WM WM
-#pragma unroll
-      for (int p = 0; p < P; ++p) acc[p] += x[p] * zr;
     }
   }
+#pragma unroll
+  for (int o = LPV / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int p = 0; p < P; ++p) acc[p] += __shfl_xor_sync(0xffffffffu, acc[p], o);
 
   // ---- beta_v | rest (Spat_Coefff, covar.cpp:142-180), production form
   const long long nk = *ch.nkept;
@@ -157,7 +268,7 @@ __global__ void __launch_bounds__(kF64Threads)
   double bnew[P], pv[NT];
 #pragma unroll
   for (int q = 0; q < NT; ++q) pv[q] = 0.0;
-  if (active) {
+  if (active && lane_v == 0) {
     double sumV[P];
 #pragma unroll
     for (int p = 0; p < P; ++p) sumV[p] = 0.0;
@@ -267,8 +378,9 @@ __global__ void __launch_bounds__(kF64Threads)
   }
   __syncthreads();
   const int nwarp = kF64Threads / 32;
-  const int lb = bm.start / kF64Threads;
-  const int nblk = max(1, (nc + kF64Threads - 1) / kF64Threads);
+  constexpr int kVox = kF64Threads / LPV;  // voxels per block
+  const int lb = bm.start / kVox;
+  const int nblk = max(1, (nc + kVox - 1) / kVox);
   if (colour == 0) {
     if (tid < P) {
       double s = 0.0;
@@ -325,13 +437,17 @@ __global__ void __launch_bounds__(kF64Threads)
 
 }  // namespace
 
-cudaError_t launch_fp64(int P, const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
-                        int nblocks, int colour, cudaStream_t st) {
+cudaError_t launch_fp64(int P, int lanes, const DatasetDev *ds, ChainDev *ch,
+                        const BlockMap *map, int nblocks, int colour, cudaStream_t st) {
   if (nblocks <= 0) return cudaSuccess;
   switch (P) {
-#define BSG_F64(PP)                                                             \
-  case PP:                                                                      \
-    fp64_colour_kernel<PP><<<nblocks, kF64Threads, 0, st>>>(ds, ch, map, colour); \
+#define BSG_F64(PP)                                                                    \
+  case PP:                                                                             \
+    if (lanes == 1)                                                                    \
+      fp64_colour_kernel<PP, 1><<<nblocks, kF64Threads, 0, st>>>(ds, ch, map, colour); \
+    else                                                                               \
+      fp64_colour_kernel<PP, kF64Lanes>                                                \
+          <<<nblocks, kF64Threads, 0, st>>>(ds, ch, map, colour);                      \
     break;
     BSG_F64(1)
     BSG_F64(2)

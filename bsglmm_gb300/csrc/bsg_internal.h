@@ -26,7 +26,8 @@ constexpr int kPostPerThread = 4;   // Omega pass (bsg_noalloc.cu)
 constexpr int kMaxThreads = 256;    // largest block of the colour kernel
 constexpr int kPredThreads = 128;   // subjects per block of the predictive pass
 constexpr int kPredWarps = 8;       // subjects (one warp each) per finishing block
-constexpr int kF64Threads = 128;    // voxels (one thread each) per FP64-chain block
+constexpr int kF64Threads = 64;     // threads of an FP64-chain block
+constexpr int kF64Lanes = 4;        // lanes per voxel of its small studies
 
 // Predictive-pass modes: after each kept sweep (ED and Qhat accumulate), on
 // demand (Mpredict of the current coefficients), or the DE deviance at the
@@ -166,10 +167,10 @@ cudaError_t prepare_fused_tc();
 cudaError_t launch_fused_wide(int P, int threads, bool wmu, const DatasetDev *ds,
                               ChainDev *ch, const BlockMap *map, int nblocks, int colour,
                               cudaStream_t st, bool pdl);
-// The colour kernel of FP64 chains (bsg_fp64.cu): one thread per voxel,
-// kF64Threads voxels per block, Philox variates, probit link.
-cudaError_t launch_fp64(int P, const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
-                        int nblocks, int colour, cudaStream_t st);
+// The colour kernel of FP64 chains (bsg_fp64.cu): `lanes` (1 or kF64Lanes)
+// lanes per voxel, blocks of kF64Threads, Philox variates, probit link.
+cudaError_t launch_fp64(int P, int lanes, const DatasetDev *ds, ChainDev *ch,
+                        const BlockMap *map, int nblocks, int colour, cudaStream_t st);
 cudaError_t launch_prb(const DatasetDev *ds, const ChainDev *ch, int chain,
                        const DatasetDev &dh, float *prb, cudaStream_t st);
 cudaError_t launch_fill(float *p, size_t n, float value, cudaStream_t st);

@@ -46,3 +46,34 @@ def test_t_sweep_matches_oracle(oracle_mod, N):
         s.run(1)
         o = oracle_mod.Problem(st.mask, st.covar, st.data, 1).chain(9, 1, model=2)
         assert np.allclose(s.beta(ch), o["beta"], rtol=TOL, atol=TOL)
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 5, 6, 31, 33, 511, 512, 513])
+def test_fp64_sweep_matches_oracle(oracle_mod, N):
+    """FP64 chains on four lanes per voxel: quads of subjects, a short last
+    pair, the 512-subject pass."""
+    import bsglmm_gb300 as bsg
+    st = synth.small_study(500 + N, shape=(6, 5, 6), N=N, P=_P(N), S=1)
+    with bsg.Sampler() as s:
+        ch = s.add_chain(s.add_dataset(st.mask, st.covar, st.data, 1), seed=11)
+        s.set_precision(ch, 64)
+        s.run(1)
+        o = oracle_mod.Problem(st.mask, st.covar, st.data, 1).chain(11, 1)
+        # FP64 on both sides: rounding, with room for the draw's conditioning
+        assert np.allclose(s.beta64(ch), o["beta"], rtol=1e-11, atol=1e-11)
+
+
+def test_fp64_one_lane_matches_oracle(oracle_mod):
+    """The same on one lane per voxel (38,912 voxels a colour and more)."""
+    import bsglmm_gb300 as bsg
+    rng = np.random.default_rng(77)
+    mask = np.ones((44, 43, 42), np.uint8)  # 39,732 voxels of each colour
+    N, V = 7, int(mask.sum())
+    covar = np.stack([np.ones(N), rng.standard_normal(N)]).astype(np.float32)
+    data = (rng.random((N, V)) < 0.2).astype(np.uint8)
+    with bsg.Sampler() as s:
+        ch = s.add_chain(s.add_dataset(mask, covar, data, 1), seed=12)
+        s.set_precision(ch, 64)
+        s.run(1)
+        o = oracle_mod.Problem(mask, covar, data, 1).chain(12, 1)
+        assert np.allclose(s.beta64(ch), o["beta"], rtol=1e-11, atol=1e-11)
