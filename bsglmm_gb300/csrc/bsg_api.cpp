@@ -313,10 +313,10 @@ bsg_status ensure_partials(bsg_ctx *ctx, int vpb) {
 // alternating (a colour kernel's early phase reads its own colour's state,
 // final once the other colour's kernel has passed its dependency point),
 // so neither colour's launch may be left out.
-void map_chain(std::vector<BlockMap> &m, int chain, int n, int vpb, int colour) {
-  (void)colour;
-  if (n == 0) m.push_back({(int32_t)chain, 0});
-  for (int s = 0; s < n; s += vpb) m.push_back({(int32_t)chain, (int32_t)s});
+void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb) {
+  if (n == 0) m.push_back({(int32_t)chain, 0, (int32_t)dataset, 0});
+  for (int s = 0; s < n; s += vpb)
+    m.push_back({(int32_t)chain, (int32_t)s, (int32_t)dataset, 0});
 }
 
 // Rebuilds the device descriptor arrays and block maps.
@@ -376,7 +376,8 @@ bsg_status build_plan(bsg_ctx *ctx) {
     // the FP64 one f64 lanes per voxel in blocks of kF64Threads
     const int gvpb = f64 ? kF64Threads / f64
                          : (mix ? ctx->threads / kMixLpv : (wmu ? ctx->threads : vpb));
-    for (int c = 0; c < 2; ++c) map_chain(g->map[c], (int)ci, (int)d.vox[c].size(), gvpb, c);
+    for (int c = 0; c < 2; ++c)
+      map_chain(g->map[c], (int)ci, ctx->ch[ci].dataset, (int)d.vox[c].size(), gvpb);
     g->vox += (double)d.V;
     g->subj_vox += (double)d.N * d.V;
     if (ctx->ch[ci].pred_on) {
@@ -389,8 +390,11 @@ bsg_status build_plan(bsg_ctx *ctx) {
         pr = &g->pred.back();
         pr->S = d.S;
       }
-      for (int t = 0; t < cv.pred_tiles; ++t) pr->pmap.push_back({(int32_t)ci, (int32_t)t});
-      for (int b = 0; b * kPredWarps < d.N; ++b) pr->fmap.push_back({(int32_t)ci, (int32_t)b});
+      const int32_t dsi = ctx->ch[ci].dataset;
+      for (int t = 0; t < cv.pred_tiles; ++t)
+        pr->pmap.push_back({(int32_t)ci, (int32_t)t, dsi, 0});
+      for (int b = 0; b * kPredWarps < d.N; ++b)
+        pr->fmap.push_back({(int32_t)ci, (int32_t)b, dsi, 0});
       pr->pchunks = std::max(pr->pchunks, (d.N + kPredThreads - 1) / kPredThreads);
     }
   }
@@ -1680,7 +1684,8 @@ bsg_status bsg_sweep_supplied(bsg_ctx *ctx, int32_t chain, const uint32_t *ubits
   // Block maps for this chain alone, one lane per voxel.
   const int thr = kParityThreads;
   std::vector<BlockMap> m[2];
-  for (int col = 0; col < 2; ++col) map_chain(m[col], chain, (int)d.vox[col].size(), thr, col);
+  for (int col = 0; col < 2; ++col)
+    map_chain(m[col], chain, c.dataset, (int)d.vox[col].size(), thr);
   e = cudaSuccess;
   BlockMap *dm0 = m[0].empty() ? nullptr : upload(ctx, m[0].data(), m[0].size(), &e);
   CK(e);

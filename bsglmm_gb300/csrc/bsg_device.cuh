@@ -351,4 +351,64 @@ __device__ __forceinline__ void solve_upper(const T (&G)[P * (P + 1) / 2],
   }
 }
 
+// The same with the diagonal's reciprocals r (rounded to nearest) at hand: a
+// quotient x / g is x r corrected once by its remainder, which rounds as the
+// division does (Markstein 1990, the theorem on correctly rounded quotients).
+__device__ __forceinline__ float div_by(float x, float g, float r) {
+  const float q = __fmul_rn(x, r);
+  return fmaf(fmaf(-q, g, x), r, q);
+}
+
+template <int P>
+__device__ __forceinline__ void solve_lower(const float (&G)[P * (P + 1) / 2],
+                                            const float (&r)[P], float (&x)[P]) {
+#pragma unroll
+  for (int a = 0; a < P; ++a) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < a; ++q) s += G[tri(a, q)] * x[q];
+    x[a] = div_by(x[a] - s, G[tri(a, a)], r[a]);
+  }
+}
+
+template <int P>
+__device__ __forceinline__ void solve_upper(const float (&G)[P * (P + 1) / 2],
+                                            const float (&r)[P], float (&x)[P]) {
+#pragma unroll
+  for (int a = P - 1; a >= 0; --a) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = a + 1; q < P; ++q) s += G[tri(q, a)] * x[q];
+    x[a] = div_by(x[a] - s, G[tri(a, a)], r[a]);
+  }
+}
+
+// -------------------------------------------------------- warp reductions --
+// Sums of N values over the warp's lanes, each by the tree of the xor
+// butterfly (lanes 16 apart first), scattered as it goes: at each step a lane
+// hands on the half of the values that it does not keep.  store(q, sum) is
+// called once per value, on the lane where it ends.
+template <int N, int O = 16, typename F>
+__device__ __forceinline__ void warp_sums(float (&v)[N], int lane, F &&store, int first = 0,
+                                          int count = N) {
+  if constexpr (O == 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i < count) store(first + i, v[i]);
+  } else {
+    constexpr int H = (N + 1) / 2;
+    const bool up = lane & O;
+    float w[H];
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const float hi = i + H < N ? v[i + H < N ? i + H : 0] : 0.f;
+      const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : hi, O);
+      w[i] = (up ? hi : v[i]) + got;
+    }
+    // (a lane may keep fewer than H values: `count` of them from `first` on)
+    warp_sums<H, O / 2>(w, lane, store, up ? first + H : first,
+                        up ? max(0, min(H, count - H)) : min(H, count));
+  }
+}
+
 }  // namespace bsg

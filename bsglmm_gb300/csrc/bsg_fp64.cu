@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kF64Threads)
 
   const BlockMap bm = map[blockIdx.x];
   ChainDev &ch = chv[bm.chain];
-  const DatasetDev &d = dsv[ch.dataset];
+  const DatasetDev &d = dsv[bm.dataset];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nc = d.n[colour];
   const int lane_v = tid % LPV;  // this lane's share of the subjects
@@ -258,7 +258,6 @@ __global__ void __launch_bounds__(kF64Threads)
     for (int p = 0; p < P; ++p) acc[p] += __shfl_xor_sync(0xffffffffu, acc[p], o);
 
   // ---- beta_v | rest (Spat_Coefff, covar.cpp:142-180), production form
-  const long long nk = *ch.nkept;
   for (int t = tid; t < P * P; t += blockDim.x) {
     Om[t] = ch.omega_d[t];
     Xtx[t] = (double)d.xtx[t];
@@ -432,7 +431,8 @@ __global__ void __launch_bounds__(kF64Threads)
     if (lane == 0) tot[q] = s;
   }
   __syncthreads();
-  if (warp == 0) wishart_warp(ch, d, tot, sweep_ll, kept, nk, 0, Supplied{}, lane);
+  if (warp == 0) wishart_warp(ch, d, tot, 0, Supplied{}, lane);
+  if (warp == 1) sweep_end_warp(ch, d, tot, sweep_ll, kept, 0, lane);
 }
 
 }  // namespace

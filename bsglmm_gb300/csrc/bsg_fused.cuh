@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
 
   const BlockMap bm = map[blockIdx.x];
   const ChainDev &ch = chv[bm.chain];
-  const DatasetDev &d = dsv[ch.dataset];
+  const DatasetDev &d = dsv[bm.dataset];
   const int tid = threadIdx.x;
   const int g = tid / LPV, k = tid % LPV;
   const int nc = d.n[colour];
@@ -613,59 +613,18 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
     }
   }
 
-  // ---- dependency protocol (programmatic dependent launch) --------------
-  // Everything above read only this colour's own coefficients, the design
-  // and the outcome bits, all final since this colour's previous launch.
-  // The beta update needs Omega and the other colour's new coefficients,
-  // written by the previous kernel in the stream: wait for its completion
-  // here, and only then let the next kernel start its own latent phase.
-  // (Without a programmatic launch both calls return at once.)
-  cudaGridDependencySynchronize();
-  cudaTriggerProgrammaticLaunchCompletion();
-  const long long nk = *ch.nkept;
-  for (int t = tid; t < P * P; t += blockDim.x) {
-    Om[t] = ch.omega_f[t];
-    Xtx[t] = d.xtx[t];
-  }
-  __syncthreads();
+  // ---- what the coefficient draw needs and no other kernel writes: the
+  // neighbour table, the normals, X'X and (colour 1) the sweep's Bartlett
+  // variates, taken before the wait below so that they are off the chain from
+  // one kernel's end to the next one's
   const bool leader = active && k == 0;
-  int err = ok ? 0 : kErrTnCap;
-  float bnew[P];   // the voxel's coefficients at the end of the sweep
-  float pv[NT];    // its Omega pair products (colour 1)
-  double wmt = 0.0;  // its term of the beta_WM conditional mean
+  int sn[6];
+  unsigned nbm = 0;
+  float e[P];
 #pragma unroll
-  for (int p = 0; p < P; ++p) bnew[p] = beta[p];
-#pragma unroll
-  for (int q = 0; q < NT; ++q) pv[q] = 0.f;
-
+  for (int t = 0; t < 6; ++t) sn[t] = leader ? d.nb[colour][(size_t)(t + 1) * nc + j] : 0;
   if (leader) {
-    // ---- beta_v | rest  (Spat_Coefff, covar.cpp:142-180) ---------------
-    float sumV[P];
-#pragma unroll
-    for (int p = 0; p < P; ++p) sumV[p] = 0.f;
-#pragma unroll
-    for (int t = 1; t <= 6; ++t) {
-      const int sn = d.nb[colour][(size_t)t * nc + j];
-#pragma unroll
-      for (int p = 0; p < P; ++p) sumV[p] += ch.beta[(size_t)p * Vp + sn];
-    }
-    const unsigned nbm = d.nbm[colour][j];
-    const float nnb = (float)__popc(nbm);
-    float b[P], Q[NT];
-#pragma unroll
-    for (int a = 0; a < P; ++a) {
-      float s = acc[a];
-#pragma unroll
-      for (int q = 0; q < P; ++q) s += Om[q + a * P] * sumV[q];
-      b[a] = s;
-#pragma unroll
-      for (int q = 0; q <= a; ++q)
-        Q[tri(a, q)] = (MIX ? qw[tri(a, q) < NQ ? tri(a, q) : 0] : Xtx[q + a * P]) +
-                       nnb * Om[q + a * P];
-    }
-    bool okc = chol_packed<P>(Q);
-
-    float e[P];
+    nbm = d.nbm[colour][j];
     if (SUPP) {
 #pragma unroll
       for (int p = 0; p < P; ++p) e[p] = __ldg(sup.normals + (size_t)v * P + p);
@@ -679,14 +638,116 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
           if (p0 + q < P) e[p0 + q] = normal_of(pick4(r, q));
       }
     }
+  }
+  if (!MIX)
+    for (int t = tid; t < P * P; t += blockDim.x) Xtx[t] = d.xtx[t];
+  const int lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const int vpb = blockDim.x / LPV;
+  const int lb = bm.start / vpb;
+  const int nblk = max(1, (nc + vpb - 1) / vpb);  // blocks of this colour
+  unsigned arrived = 0;
+  if (colour == 0) {
+    // every thread of the block has read this colour's count
+    if (tid == 0) arrived = atomicInc(ch.done, (unsigned)(nblk - 1));
+  } else if (!SUPP && lb == nblk - 1 && warp == nwarp - 1) {
+    // the Bartlett variates (they do not depend on S), by the last warp, which
+    // mostly has no voxels; its previous reader, the last colour-1 launch,
+    // has completed
+    const int er = __reduce_or_sync(0xffffffffu, wishart_draws(ch, d, sweep_ll, lane, ch.wdraw));
+    if (er && lane == 0) {
+      atomicOr(ch.status, er);
+      atomicOr(ch.any_status, er);
+    }
+  }
+
+  // ---- dependency protocol (programmatic dependent launch) --------------
+  // Everything above read only this colour's own coefficients, the design
+  // and the outcome bits, all final since this colour's previous launch.
+  // The beta update needs Omega and the other colour's new coefficients,
+  // written by the previous kernel in the stream: wait for its completion
+  // here, and only then let the next kernel start its own latent phase.
+  // (Without a programmatic launch both calls return at once.)
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  static_assert(kMaxP * kMaxP <= 64, "one entry of Omega per thread");
+  if (tid < P * P) Om[tid] = ch.omega_f[tid];
+  float sumV[P];
+#pragma unroll
+  for (int p = 0; p < P; ++p) sumV[p] = 0.f;
+  if (leader) {
+#pragma unroll
+    for (int t = 0; t < 6; ++t)
+#pragma unroll
+      for (int p = 0; p < P; ++p) sumV[p] += ch.beta[(size_t)p * Vp + sn[t]];
+  }
+  __syncthreads();
+  // The probit Q = X'X + n_v Omega has one value per neighbour count n_v: the
+  // first seven threads factor them (G with the reciprocals of its diagonal
+  // behind it) for the block's voxels.
+  constexpr int GN = NT + P;
+  __shared__ float Gf[MIX ? 1 : 7][MIX ? 1 : GN];
+  __shared__ int Gok[7];
+  if constexpr (!MIX) {
+    if (tid < 7) {
+      float Q[NT];
+#pragma unroll
+      for (int a = 0; a < P; ++a)
+#pragma unroll
+        for (int q = 0; q <= a; ++q)
+          Q[tri(a, q)] = Xtx[q + a * P] + (float)tid * Om[q + a * P];
+      Gok[tid] = chol_packed<P>(Q);
+#pragma unroll
+      for (int q = 0; q < NT; ++q) Gf[tid][q] = Q[q];
+#pragma unroll
+      for (int a = 0; a < P; ++a) Gf[tid][NT + a] = 1.f / Q[tri(a, a)];
+    }
+    __syncthreads();
+  }
+  int err = ok ? 0 : kErrTnCap;
+  float bnew[P];   // the voxel's coefficients at the end of the sweep
+  float pv[NT];    // its Omega pair products (colour 1)
+  double wmt = 0.0;  // its term of the beta_WM conditional mean
+#pragma unroll
+  for (int p = 0; p < P; ++p) bnew[p] = beta[p];
+#pragma unroll
+  for (int q = 0; q < NT; ++q) pv[q] = 0.f;
+
+  if (leader) {
+    // ---- beta_v | rest  (Spat_Coefff, covar.cpp:142-180) ---------------
+    const int nnb = __popc(nbm);
+    float b[P], Q[NT], rd[P];
+#pragma unroll
+    for (int a = 0; a < P; ++a) {
+      float s = acc[a];
+#pragma unroll
+      for (int q = 0; q < P; ++q) s += Om[q + a * P] * sumV[q];
+      b[a] = s;
+    }
+    bool okc;
+    if constexpr (MIX) {
+#pragma unroll
+      for (int a = 0; a < P; ++a)
+#pragma unroll
+        for (int q = 0; q <= a; ++q)
+          Q[tri(a, q)] = qw[tri(a, q) < NQ ? tri(a, q) : 0] + (float)nnb * Om[q + a * P];
+      okc = chol_packed<P>(Q);
+#pragma unroll
+      for (int a = 0; a < P; ++a) rd[a] = 1.f / Q[tri(a, a)];
+    } else {
+      okc = Gok[nnb];
+#pragma unroll
+      for (int q = 0; q < NT; ++q) Q[q] = Gf[nnb][q];
+#pragma unroll
+      for (int a = 0; a < P; ++a) rd[a] = Gf[nnb][NT + a];
+    }
 
     float out[P];
     if (!SUPP || sup.form == 1) {
       // Q = G G':  m = G^-T G^-1 b,  beta = m + G^-T e = G^-T (G^-1 b + e)
-      solve_lower<P>(Q, b);
+      solve_lower<P>(Q, rd, b);
 #pragma unroll
       for (int p = 0; p < P; ++p) out[p] = b[p] + e[p];
-      solve_upper<P>(Q, out);
+      solve_upper<P>(Q, rd, out);
     } else {
       // Reference draw (covar.cpp:168-177): V = Q^-1 by columns
       // (cholesky_invert_float), m = V b, L = chol(V), beta = m + L e.
@@ -696,8 +757,8 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         float x[P];
 #pragma unroll
         for (int q = 0; q < P; ++q) x[q] = (q == kk) ? 1.f : 0.f;
-        solve_lower<P>(Q, x);
-        solve_upper<P>(Q, x);
+        solve_lower<P>(Q, rd, x);
+        solve_upper<P>(Q, rd, x);
 #pragma unroll
         for (int q = 0; q < P; ++q) Vc[kk][q] = x[q];
       }
@@ -746,19 +807,22 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
       wmt = (double)wmv * (sz + (double)d.N * (double)bwm - sxb);
     }
 
-    // ---- posterior running sums of the kept sweep (mcmc.cpp:637-645) --
+    // ---- posterior running sums of the kept sweep (mcmc.cpp:637-645): only
+    // this thread adds to these entries, by reductions at the L2 that it
+    // does not wait for (the same FP64 additions as a load, add and store)
     if (kept) {
 #pragma unroll
       for (int p = 0; p < P; ++p) {
         const double x = (double)bnew[p];
-        ch.acc_sum[(size_t)p * d.V + v] += x;
-        ch.acc_sq[(size_t)p * d.V + v] += x * x;
+        atomicAdd(ch.acc_sum + (size_t)p * d.V + v, x);
+        atomicAdd(ch.acc_sq + (size_t)p * d.V + v, x * x);
       }
 #pragma unroll
       for (int g2 = 0; g2 < P; ++g2)
         if (g2 < d.S)
-          ch.prb_sum[(size_t)g2 * d.V + v] +=
-              (double)(MIX ? prob_logit(bnew[g2], ch.inv_lf) : prob_sdnorm(bnew[g2] + bwm));
+          atomicAdd(ch.prb_sum + (size_t)g2 * d.V + v,
+                    (double)(MIX ? prob_logit(bnew[g2], ch.inv_lf)
+                                 : prob_sdnorm(bnew[g2] + bwm)));
     }
 
     // ---- Omega pair products (Spat_Coef_Prec, covarGPU.cu:953-1013) -----
@@ -770,14 +834,13 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
     if (colour == 1) {
 #pragma unroll
       for (int t = 0; t < 6; ++t) {
-        const int sn = d.nb[1][(size_t)(t + 1) * nc + j];
         const bool fwd = t & 1;
         const bool nin = (nbm >> t) & 1u;
         float dd[P];
         bool ind[P];
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-          const float bn = ch.beta[(size_t)p * Vp + sn];
+          const float bn = ch.beta[(size_t)p * Vp + sn[t]];
           dd[p] = bnew[p] - bn;
           ind[p] = fwd ? (bn != 0.f) : (nin && bnew[p] != 0.f);
         }
@@ -803,124 +866,123 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
   __shared__ double red[kMaxThreads / 32][kFusedVals];
   __shared__ double tot[kFusedVals];
   __shared__ int is_last;
-  const int lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
   constexpr int kColOff = kMaxPairs;
   constexpr int NV = NT + P + (WMU ? 1 : 0);  // values reduced per block
   // The pair products and coefficients of a warp's 32 voxels are summed in
-  // FP32 by a fixed shuffle tree (this part's FP64 pipe does two lanes per
-  // clock per SM: an FP64 tree over all 24 resident warps took about 15 us
-  // per colour-1 launch), then in FP64 across warps and blocks; the beta_WM
-  // term stays FP64 throughout.
+  // FP32 by a fixed tree over the lanes that scatters the values as it goes
+  // (warp_sums: P = 5 takes 21 shuffles for its 20 values, not 100), then in
+  // FP64 across warps and blocks; the beta_WM term stays FP64 throughout.
+  // (This part's FP64 pipe does two lanes per clock per SM.)
+  if (colour == 0) {
+    float vals[P];
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    if (colour == 0 && q < NT) continue;
-    double val;
-    if (q < NT + P) {
-      float f = q < NT ? pv[q] : bnew[q - NT];
+    for (int p = 0; p < P; ++p) vals[p] = bnew[p];
+    warp_sums<P>(vals, lane, [&](int q, float f) { red[warp][kColOff + q] = (double)f; });
+  } else {
+    float vals[NT + P];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
-      val = (double)f;
-    } else {
-      val = wmt;
+    for (int q = 0; q < NT; ++q) vals[q] = pv[q];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
-    }
-    if (lane == 0)
-      red[warp][q < NT ? q : (q < NT + P ? kColOff + (q - NT) : kWmOff)] = val;
+    for (int p = 0; p < P; ++p) vals[NT + p] = bnew[p];
+    warp_sums<NT + P>(vals, lane, [&](int q, float f) {
+      red[warp][q < NT ? q : kColOff + (q - NT)] = (double)f;
+    });
+  }
+  if constexpr (WMU) {
+    double val = wmt;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
+    if (lane == 0) red[warp][kWmOff] = val;
   }
   __syncthreads();
-  const int vpb = blockDim.x / LPV;
-  const int lb = bm.start / vpb;
-  const int nblk = max(1, (nc + vpb - 1) / vpb);  // blocks of this colour
-  // Sum of one value over the blocks' partials (value-major, so a warp
-  // reads consecutive blocks) in a fixed order, so the draw is bitwise
-  // reproducible: lane l loads the blocks l, l + 32, ... of a 512-block
-  // chunk together and adds them as a tree, then the lanes are combined.
-  auto rows = [&](const double *base, int nrow) -> double {
-    double s = 0.0;
-    for (int c0 = 0; c0 < nrow; c0 += 512) {
-      double v[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int r = c0 + lane + 32 * u;
-        v[u] = r < nrow ? __ldcg(base + r) : 0.0;
-      }
-#pragma unroll
-      for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-        for (int u = 0; u < w; ++u) v[u] += v[u + w];
-      s += v[0];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  // value q over the block's warps, as a tree of pairs, fours and eights: so
+  // blocks of 64 and 128 threads give rows that combine to the same sums as
+  // blocks of 256 (`rows` below)
+  auto block_sum = [&](int q) -> double {
+    double s = red[0][q];
+    if (nwarp >= 2) s += red[1][q];
+    if (nwarp >= 4) s += red[2][q] + red[3][q];
+    if (nwarp >= 8) s += (red[4][q] + red[5][q]) + (red[6][q] + red[7][q]);
     return s;
   };
   if (colour == 0) {
-    if (tid < P || (WMU && tid == kMaxP)) {
-      const int q = tid < P ? kColOff + tid : kWmOff;
-      double s = 0.0;
-      for (int w = 0; w < nwarp; ++w) s += red[w][q];
-      ch.partials0[(size_t)tid * ch.pstride0 + lb] = s;
-      __threadfence();
-    }
-    __syncthreads();
-    if (tid == 0) is_last = atomicAdd(ch.done, 1u) == (unsigned)(nblk - 1);
-    __syncthreads();
-    if (!is_last) return;
-    // The last colour-0 block sums the column sums (and the beta_WM term)
-    // over the colour's blocks while colour 1 starts, and advances this
-    // colour's count.
-    __threadfence();
-    for (int m = warp; m < P + (WMU ? 1 : 0); m += nwarp) {
-      const int q = m < P ? m : kMaxP;
-      const double s = rows(ch.partials0 + (size_t)q * ch.pstride0, nblk);
-      if (lane == 0) ch.tot0[q] = s;
-    }
-    // the sweep's Bartlett variates (they do not depend on S), for the
-    // Omega draw at the end of colour 1
-    if (!SUPP && warp == nwarp - 1) {
-      const int e = __reduce_or_sync(0xffffffffu, wishart_draws(ch, d, sweep_ll, lane, ch.wdraw));
-      if (e && lane == 0) {
-        atomicOr(ch.status, e);
-        atomicOr(ch.any_status, e);
-      }
-    }
-    if (tid == 0) {
-      ch.sweep[0] = sweep_ll + 1;
-      ch.done[0] = 0u;
-      __threadfence();
-    }
+    if (tid < P || (WMU && tid == kMaxP))
+      ch.partials0[(size_t)tid * ch.pstride0 + lb] = block_sum(tid < P ? kColOff + tid : kWmOff);
+    // the last block to have read this colour's count advances it
+    if (tid == 0 && arrived == (unsigned)(nblk - 1)) ch.sweep[0] = sweep_ll + 1;
     return;
   }
   if (tid < kFusedVals) {
     const bool live =
         tid < kMaxPairs ? tid < NT : ((WMU && tid == kWmOff) || (tid - kColOff) < P);
-    if (live) {
-      double s = 0.0;
-      for (int w = 0; w < nwarp; ++w) s += red[w][tid];
-      ch.partials1[(size_t)tid * ch.pstride1 + lb] = s;
-      __threadfence();
-    }
+    if (live) ch.partials1[(size_t)tid * ch.pstride1 + lb] = block_sum(tid);
   }
   __syncthreads();
   if (tid == 0) {
-    const unsigned prev = atomicAdd(ch.done + 1, 1u);
-    is_last = prev == (unsigned)(nblk - 1);
+    __threadfence();  // the block's rows (ordered by the barrier) before the arrival
+    is_last = atomicInc(ch.done + 1, (unsigned)(nblk - 1)) == (unsigned)(nblk - 1);
+    __threadfence();
   }
   __syncthreads();
   if (!is_last) return;
-  __threadfence();
-  // warp w takes the live values m = w, w + nwarp, ...; colour 0's totals
-  // (final since that kernel completed) are added to the column sums
-  for (int m = warp; m < NV; m += nwarp) {
+  // Sums of the values over the blocks' rows (value-major) in a fixed order,
+  // so the draw is bitwise reproducible: the rows of 256 threads' worth of
+  // warps first (a tile, the same for every block size), then the tiles over
+  // the lanes that share a value, colour 1's and (column sums, beta_WM)
+  // colour 0's, then the lanes.  An FP64 instruction takes 16 cycles of the
+  // SM's pipe whatever the number of its lanes: up to 64 tiles eight lanes
+  // share a value and a warp takes four (7 tiles, P = 3; 2.8 us with
+  // 32 lanes each), beyond it is the loads in flight that count (450 tiles, P
+  // = 5: eight per lane, 32 lanes).
+  const int sub = kMaxThreads / blockDim.x;
+  const int ntile = (nblk + sub - 1) / sub;
+  const int nblk0 = max(1, (d.n[0] + vpb - 1) / vpb), ntile0 = (nblk0 + sub - 1) / sub;
+  auto tile = [&](const double *base, int nrow, int nt, int r) -> double {
+    auto ld = [&](int i) -> double { return i < nrow ? __ldcg(base + i) : 0.0; };
+    if (r >= nt) return 0.0;
+    if (sub == 1) return ld(r);
+    if (sub == 2) return ld(2 * r) + ld(2 * r + 1);
+    return (ld(4 * r) + ld(4 * r + 1)) + (ld(4 * r + 2) + ld(4 * r + 3));
+  };
+  const bool few = ntile <= 64;
+  const int vw = few ? 4 : 1, ln = 32 / vw;  // values per warp, lanes per value
+  auto rows = [&](const double *base, int nrow, int nt, double s) -> double {
+    if (few) {
+      for (int r = lane & 7; r < nt; r += 32) {
+        const double x0 = tile(base, nrow, nt, r), x1 = tile(base, nrow, nt, r + 8);
+        const double x2 = tile(base, nrow, nt, r + 16), x3 = tile(base, nrow, nt, r + 24);
+        s += x0;
+        if (r + 8 < nt) s += x1;
+        if (r + 16 < nt) s += x2;
+        if (r + 24 < nt) s += x3;
+      }
+    } else {
+      for (int r = lane; r < nt; r += 256) {
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = tile(base, nrow, nt, r + 32 * u);
+#pragma unroll
+        for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+          for (int u = 0; u < w; ++u) x[u] += x[u + w];
+        s += x[0];
+      }
+    }
+    return s;
+  };
+  for (int m0 = vw * warp; m0 < NV; m0 += vw * nwarp) {
+    const int mine = m0 + lane / ln, m = min(mine, NV - 1);
     const int q = m < NT ? m : (m < NT + P ? kColOff + (m - NT) : kWmOff);
-    double s = rows(ch.partials1 + (size_t)q * ch.pstride1, nblk);
-    if (q >= kColOff) s += __ldcg(ch.tot0 + (q == kWmOff ? kMaxP : q - kColOff));
-    if (lane == 0) tot[q] = s;
+    double s = rows(ch.partials1 + (size_t)q * ch.pstride1, nblk, ntile, 0.0);
+    if (m >= NT)
+      s = rows(ch.partials0 + (size_t)(m < NT + P ? m - NT : kMaxP) * ch.pstride0, nblk0,
+               ntile0, s);
+    for (int o = ln / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane % ln == 0 && mine < NV) tot[q] = s;
   }
   __syncthreads();
-  if (warp == 0)
-    wishart_warp(ch, d, tot, (long long)sweep_ll, kept, nk, SUPP ? 1 : 0, sup, lane);
+  if (warp == 0) wishart_warp(ch, d, tot, SUPP ? 1 : 0, sup, lane);
+  if (warp == 1) sweep_end_warp(ch, d, tot, sweep_ll, kept, SUPP ? 1 : 0, lane);
 }
 
 // Launch of one instantiation; with pdl the launch carries the

@@ -137,7 +137,9 @@ struct Supplied {
 
 struct BlockMap {
   int32_t chain;
-  int32_t start;  // first colour position (fused) or merged position (post)
+  int32_t start;    // first colour position (fused) or merged position (post)
+  int32_t dataset;  // the chain's (colour kernels: one dependent load less)
+  int32_t pad;
 };
 
 // ---- launchers (bsg_kernels.cu) ----------------------------------------

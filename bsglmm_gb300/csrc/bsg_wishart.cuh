@@ -61,6 +61,17 @@ static __device__ int wishart_draws(const ChainDev &ch, const DatasetDev &d,
   return err;
 }
 
+// 1 / sqrt(d) in FP64 from the single-precision value (relative error e of
+// some 2^-22) by one third-order step, which leaves e^3: four dependent FP64
+// operations, each about 80 cycles here; rounds within an ulp or so.  (d, a
+// pivot of S + I, is hardly ever outside a float's range.)
+static __device__ __forceinline__ double rsqrt_step(double d) {
+  if (!(d > 1e-30 && d < 1e30)) return rsqrt(d);
+  const double y = (double)rsqrt_approx((float)d);
+  const double e = fma(-(d * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
 // Omega | beta ~ Wishart(df, (S + I)^-1) by the Bartlett construction of
 // rwishart2 (cholesky.cpp:245-286), FP64, one warp.  The reference forms
 // chol((S + I)^-1) by chol -> invert -> chol (covar.cpp:286-291,
@@ -70,12 +81,10 @@ static __device__ int wishart_draws(const ChainDev &ch, const DatasetDev &d,
 // diagonal, so chol((S + I)^-1) = U^-T (the Cholesky factor is unique),
 // and B = U^-T T comes from forward substitution without forming U^-T.
 static __device__ void wishart_warp(const ChainDev &ch, const DatasetDev &d,
-                                    const double *tot, long long sweep,
-                                    bool kept, long long nk, int supplied,
+                                    const double *tot, int supplied,
                                     const Supplied &sup, int lane) {
   __shared__ double A[kMaxP][kMaxP], T[kMaxP][kMaxP], B[kMaxP][kMaxP], rd[kMaxP];
   const int P = d.P;
-  const uint32_t cid = ch.chain_id << 8, sw = (uint32_t)sweep;
   int err = 0;
   // entry q of the packed lower triangle is (r, c), r >= c; the lanes take
   // the entries (one round up to P = 7), so that every stage below is a
@@ -100,7 +109,7 @@ static __device__ void wishart_warp(const ChainDev &ch, const DatasetDev &d,
   for (int k = P - 1; k >= 0; --k) {
     const double dk = A[k][k];
     ok = ok && (dk > 0.0);
-    const double rs = rsqrt(dk);
+    const double rs = rsqrt_step(dk);
     __syncwarp();
     if (lane < k) A[lane][k] = A[k][lane] * rs;
     if (lane == k) {
@@ -174,7 +183,20 @@ static __device__ void wishart_warp(const ChainDev &ch, const DatasetDev &d,
   } else {
     err |= kErrWishart;
   }
-  if (lane < P) ch.colmean[lane] = (float)(tot[kMaxPairs + lane] / (double)d.V);
+  err = __reduce_or_sync(0xffffffffu, err);
+  if (lane == 0 && err) {
+    atomicOr(ch.status, err);
+    atomicOr(ch.any_status, err);
+  }
+}
+
+// What else ends a sweep and does not wait for Omega, run by another warp
+// beside wishart_warp: the column means, beta_WM, the counters.
+static __device__ void sweep_end_warp(const ChainDev &ch, const DatasetDev &d,
+                                      const double *tot, long long sweep, bool kept,
+                                      int supplied, int lane) {
+  const uint32_t cid = ch.chain_id << 8, sw = (uint32_t)sweep;
+  if (lane < d.P) ch.colmean[lane] = (float)(tot[kMaxPairs + lane] / (double)d.V);
   if (lane == 0) {
     // beta_WM | Z, beta ~ N(var * sum_v WM_v sum_i (Z_iv - x_i' beta_v),
     // var = 1 / (N sum_v WM_v^2)) (updateBetaGPU, covarGPU.cu:680-720)
@@ -188,21 +210,16 @@ static __device__ void wishart_warp(const ChainDev &ch, const DatasetDev &d,
         bw = nb;
         *ch.wm_beta = nb;
       } else {
-        err |= kErrNaN;
+        atomicOr(ch.status, kErrNaN);
+        atomicOr(ch.any_status, kErrNaN);
       }
     }
-    if (kept) *ch.wm_sum += (double)bw;  // MWM of mcmc.cpp:636
-  }
-  err = __reduce_or_sync(0xffffffffu, err);
-  if (lane == 0) {
-    if (err) {
-      atomicOr(ch.status, err);
-      atomicOr(ch.any_status, err);
+    if (kept) {
+      *ch.wm_sum += (double)bw;  // MWM of mcmc.cpp:636
+      *ch.nkept += 1;
     }
     ch.sweep[1] = sweep + 1;
-    if (kept) *ch.nkept = nk + 1;
     ch.done[1] = 0u;
-    __threadfence();
   }
 }
 
