@@ -49,6 +49,9 @@ struct Group {
                         // no early start); 0: FP32
   bool wide = false;    // the 16-subject whole-word step (bsg_fused_wide.cu)
   double vox = 0, subj_vox = 0;  // its chains' voxels and N x voxels
+  int threads = 256;             // per block
+  bool early = true;             // its kernels start early (programmatic launch)
+  std::vector<int> chains;
   std::vector<BlockMap> map[2];
   BlockMap *d_map[2] = {nullptr, nullptr};
   // predictive pass of the group's chains that have it on, one launch pair
@@ -103,6 +106,7 @@ struct bsg_ctx {
   std::vector<Group> groups;
   int *any_status = nullptr;  // device word: OR of every chain's error bits
   int lpv = 1, threads = 256;
+  bool threads_set = false;  // by bsg_set_tuning; else chosen per group
   bool tc = false;  // probit X'Z on the tensor cores (BF16x3 split)
   int step = 0;     // subjects per whole-word step: 8, 16, 0 = chosen per group
 #ifdef BSG_NO_PDL
@@ -274,12 +278,15 @@ int f64_lanes(const Dataset &d) {
 // (value-major, so that the last block's sums read consecutive blocks):
 // column sums (colour 0) and pairs + column sums (colour 1), sized for the
 // smallest tile the context launches; tot0 takes colour 0's totals.
-bsg_status ensure_partials(bsg_ctx *ctx, int vpb) {
+bsg_status ensure_partials(bsg_ctx *ctx) {
   cudaError_t e;
-  const int vpb32 = vpb;
   for (auto &c : ctx->ch) {
     const Dataset &d = ctx->ds[c.dataset];
-    const int vpb = c.dev.fp64 ? std::min(vpb32, kF64Threads / f64_lanes(d)) : vpb32;
+    const int thr = std::min(ctx->threads, kSmallBlock);
+    const int vpb = c.dev.fp64 ? std::min(kParityThreads, kF64Threads / f64_lanes(d))
+                    : c.dev.model != 1
+                        ? std::min(kParityThreads, thr / kMixLpv)
+                        : std::min(kParityThreads, c.dev.wm_update ? thr : thr / ctx->lpv);
     const size_t n0 = std::max<size_t>(1, (d.vox[0].size() + vpb - 1) / vpb);
     const size_t n1 = std::max<size_t>(1, (d.vox[1].size() + vpb - 1) / vpb);
     if (n0 > c.cap0) {
@@ -319,6 +326,42 @@ void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb)
     m.push_back({(int32_t)chain, (int32_t)s, (int32_t)dataset, 0});
 }
 
+// Threads per block of a group's colour kernels: 256, or 128 where that leaves
+// the busiest SM fewer warps (grids of one wave: 77 blocks of 256 put eight
+// warps on half of the SMs, 152 of 128 four on each) and the subjects are
+// enough for that to count.  Measured, us per sweep with 256 / 128 threads,
+// P = 4: 38,456 voxels (151 blocks of 128) N = 60 25.7 / 29.4, N = 120 30.9 /
+// 33.2, N = 200 44.7 / 38.9, N = 350 73.4 / 55.6; 20,672 voxels N = 120 29.9 /
+// 28.9; 84,368 (165 blocks of 256) N = 120 48.6 / 51.2, N = 200 73.8 / 61.2;
+// 40,008 (157 blocks of 128, two on five SMs) N = 350 73.6 / 74.4.  The t and
+// logistic links (two lanes per voxel) cost three to four times as much a
+// subject: 8,552 voxels N = 60 50.2 / 46.6, 40,008 voxels N = 301 188 / 164.
+// The sums combine in one order, so the results do not depend on it.
+int group_threads(const Group &g, int64_t b256, int64_t b128, int nsm, int threads, bool set) {
+  if (set || threads != kMaxThreads) return threads;
+  const int64_t w256 = 8 * ((b256 + nsm - 1) / nsm), w128 = 4 * ((b128 + nsm - 1) / nsm);
+  // P > 5 t/logit: three blocks of 128 threads fit an SM, or one of 256 (with
+  // more registers a thread); the latter is better where it fills each SM once
+  if (g.mix && g.P > 5) return w256 <= 8 && w128 >= 8 ? kMaxThreads : kSmallBlock;
+  if (w256 > 16 || w128 >= w256) return kMaxThreads;
+  const double least = g.mix ? 32.0 : w256 <= 8 ? 150.0 : 160.0;
+  return g.subj_vox >= least * g.vox ? kSmallBlock : kMaxThreads;
+}
+
+// The whole-word step of a probit / beta_WM group (one lane per voxel): 16
+// subjects (four Philox calls at two resident blocks) where the voxel's
+// latent work dominates (P > 5, or N >= 384 on average) or two blocks per SM
+// take no more waves than three, else 8 subjects at three blocks; the results
+// are the same either way.  Measured, us per sweep with 8 / 16: N = 1000, P =
+// 5 6.5 % less; 290,369 voxels (567 blocks) N = 50 90 / 81, N = 300 240 / 221;
+// N = 50, P = 3 chains of 7 blocks: 32 of them 33 / 29, 64 (448 blocks) 44 /
+// 55, 80 69 / 57, 128 81 / 91, 200 121 / 137.
+bool group_wide(const Group &g, int64_t b256, int nsm) {
+  constexpr int kWideMinN = 384;
+  const int64_t w2 = (b256 + 2 * nsm - 1) / (2 * nsm), w3 = (b256 + 3 * nsm - 1) / (3 * nsm);
+  return g.P > 5 || g.subj_vox >= (double)kWideMinN * g.vox || w2 <= w3;
+}
+
 // Rebuilds the device descriptor arrays and block maps.
 bsg_status build_plan(bsg_ctx *ctx) {
   if (ctx->plan_valid) return BSG_OK;
@@ -337,10 +380,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
     ctx->d_ch = (ChainDev *)dalloc(ctx, sizeof(ChainDev) * ctx->d_ch_cap, &e);
     CK(e);
   }
-  const int vpb = ctx->threads / ctx->lpv;
-  // partial rows for the smallest tile any kernel of this context uses
-  bsg_status ps = ensure_partials(
-      ctx, std::min({vpb, kParityThreads, ctx->threads / kMixLpv}));
+  bsg_status ps = ensure_partials(ctx);
   if (ps) return ps;
   std::vector<DatasetDev> hds;
   for (auto &d : ctx->ds) hds.push_back(d.dev);
@@ -372,12 +412,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
       g->wm_any = wmu;
       g->fp64 = f64;
     }
-    // the t/logit kernel runs kMixLpv lanes per voxel, the beta_WM one one,
-    // the FP64 one f64 lanes per voxel in blocks of kF64Threads
-    const int gvpb = f64 ? kF64Threads / f64
-                         : (mix ? ctx->threads / kMixLpv : (wmu ? ctx->threads : vpb));
-    for (int c = 0; c < 2; ++c)
-      map_chain(g->map[c], (int)ci, ctx->ch[ci].dataset, (int)d.vox[c].size(), gvpb);
+    g->chains.push_back((int)ci);
     g->vox += (double)d.V;
     g->subj_vox += (double)d.N * d.V;
     if (ctx->ch[ci].pred_on) {
@@ -398,23 +433,37 @@ bsg_status build_plan(bsg_ctx *ctx) {
       pr->pchunks = std::max(pr->pchunks, (d.N + kPredThreads - 1) / kPredThreads);
     }
   }
-  // The whole-word step of each probit / beta_WM group (one lane per
-  // voxel): 16 subjects (four Philox calls at two resident blocks) where the
-  // voxel's latent work dominates (P > 5, or N >= kWideMinN on average) or
-  // the grid leaves SMs room (at most two blocks per SM), else 8 subjects
-  // at three blocks; the results are the same either way.  Measured: the
-  // 16-subject step is 6.5 % faster per sweep at N = 1000, P = 5 and 3.5 %
-  // at N = 500, P = 6 (1.5M voxels); groups of 64 replicate studies with
-  // N of 210-300 on average ran 2 % slower on it than on the 8-subject step.
-  constexpr int kWideMinN = 384;
   int nsm = 0;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
   for (auto &g : ctx->groups) {
+    // the t/logit kernel runs kMixLpv lanes per voxel, the beta_WM one one,
+    // the FP64 one g.fp64 lanes per voxel in blocks of kF64Threads
+    const int lanes = g.fp64 ? g.fp64 : g.mix ? kMixLpv : g.wm_any ? 1 : ctx->lpv;
+    auto blocks = [&](int threads) -> int64_t {
+      int64_t n[2] = {0, 0};
+      for (int ci : g.chains)
+        for (int c = 0; c < 2; ++c)
+          n[c] += std::max<int64_t>(1, ((int64_t)ctx->ds[ctx->ch[ci].dataset].vox[c].size() *
+                                            lanes + threads - 1) / threads);
+      return std::max(n[0], n[1]);
+    };
+    g.threads = g.fp64 ? kF64Threads
+                       : group_threads(g, blocks(kMaxThreads), blocks(kSmallBlock), nsm,
+                                       ctx->threads, ctx->threads_set);
+    // A t/logit grid of up to one block per SM with much work per voxel waits
+    // for the kernel before it: started early, beside the blocks of that one,
+    // two of its own can come to share an SM, which costs more than the overlap
+    // gives (38,456 voxels, 151 blocks, N = 1200, P = 3 logistic: 597 us per
+    // sweep early, 506 after).  (Above P = 5 an SM has room for one only.)
+    g.early = !(g.mix && g.P <= 5 && g.threads == kMaxThreads && blocks(kMaxThreads) <= nsm &&
+                g.subj_vox >= 256.0 * g.vox);
     const bool eligible = !g.mix && !g.fp64 && (g.wm_any || (ctx->lpv == 1 && !ctx->tc));
-    const bool fits = (int64_t)std::max(g.map[0].size(), g.map[1].size()) <= 2 * (int64_t)nsm;
-    const bool auto_wide =
-        g.P > 5 || g.subj_vox >= (double)kWideMinN * g.vox || fits;
-    g.wide = eligible && (ctx->step == 16 || (ctx->step == 0 && auto_wide));
+    g.wide = eligible && (ctx->step == 16 ||
+                          (ctx->step == 0 && group_wide(g, blocks(kMaxThreads), nsm)));
+    for (int ci : g.chains)
+      for (int c = 0; c < 2; ++c)
+        map_chain(g.map[c], ci, ctx->ch[ci].dataset,
+                  (int)ctx->ds[ctx->ch[ci].dataset].vox[c].size(), g.threads / lanes);
   }
   for (auto &g : ctx->groups) {
     for (int c = 0; c < 2; ++c) {
@@ -449,19 +498,19 @@ cudaError_t launch_colour(bsg_ctx *ctx, const Group &g, int c, cudaStream_t st, 
     return launch_fp64(g.P, g.fp64, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
                        st);
   if (g.mix)
-    return launch_fused_mix(g.P, ctx->threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
+    return launch_fused_mix(g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
                             (int)g.map[c].size(), c, st, pdl);
   if (g.wide)
-    return launch_fused_wide(g.P, ctx->threads, g.wm_any, ctx->d_ds, ctx->d_ch, g.d_map[c],
+    return launch_fused_wide(g.P, g.threads, g.wm_any, ctx->d_ds, ctx->d_ch, g.d_map[c],
                              (int)g.map[c].size(), c, st, pdl);
   if (g.wm_any)
-    return launch_fused_wm(g.P, ctx->threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
+    return launch_fused_wm(g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
                            (int)g.map[c].size(), c, st, pdl);
   if (ctx->tc && ctx->lpv == 1)
-    return launch_fused_tc(g.P, ctx->threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
+    return launch_fused_tc(g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
                            (int)g.map[c].size(), c, st, pdl);
   const Supplied sup{};
-  return launch_fused(g.P, ctx->lpv, ctx->threads, false, ctx->d_ds, ctx->d_ch,
+  return launch_fused(g.P, ctx->lpv, g.threads, false, ctx->d_ds, ctx->d_ch,
                       g.d_map[c], (int)g.map[c].size(), c, sup, st, pdl);
 }
 
@@ -470,7 +519,7 @@ cudaError_t enqueue_group(bsg_ctx *ctx, const Group &g, cudaStream_t st) {
   for (int c = 0; c < 2; ++c) {
     // the colour-0 latent phase reads beta_WM, which the previous colour-1
     // kernel draws when the update is on: no early start then
-    const bool pdl = ctx->pdl && !(c == 0 && g.wm_any) && !g.fp64;
+    const bool pdl = ctx->pdl && g.early && !(c == 0 && g.wm_any) && !g.fp64;
     e = launch_colour(ctx, g, c, st, pdl);
     if (e != cudaSuccess) return e;
   }
@@ -930,9 +979,11 @@ bsg_status bsg_set_tuning(bsg_ctx *ctx, int32_t lanes_per_voxel,
   if (!fused_supported(1, lpv, thr))
     return fail(ctx, BSG_ERR_UNSUPPORTED,
                 "lanes_per_voxel in {1,2,4,8}, block_threads in {64,128,256}");
-  if (lpv != ctx->lpv || thr != ctx->threads) {
+  const bool set = ctx->threads_set || block_threads;
+  if (lpv != ctx->lpv || thr != ctx->threads || set != ctx->threads_set) {
     ctx->lpv = lpv;
     ctx->threads = thr;
+    ctx->threads_set = set;
     ctx->plan_valid = false;
   }
   return BSG_OK;

@@ -43,7 +43,7 @@ constexpr int fused_min_blocks() {
   return BSG_FUSED_MIN_BLOCKS;
 #else
   // the t/logit kernel also keeps the voxel's X' Phi X in registers
-  return MIX ? (P <= 5 ? 2 : 1) : ((WIDE || P > 5) ? 2 : 3);
+  return MIX ? (P <= 5 ? 2 : (WIDE ? 3 : 1)) : ((WIDE || P > 5) ? 2 : 3);
 #endif
 }
 
@@ -56,17 +56,19 @@ constexpr int fused_min_blocks() {
 // term of its conditional mean through the block partials.
 // TC: the probit kernel's X'(Z - b_WM WM) on the tensor cores as a BF16x3
 // split product (bsg_mma.cuh), one lane per voxel; the rest is unchanged.
-// WIDE: the 16-subject whole-word step (identical results).
+// WIDE: the 16-subject whole-word step (identical results); for the t/logit
+// links above P = 5, the form for blocks of 128 threads.
 template <int P, int LPV, bool SUPP, bool MIX = false, bool WMU = false, bool TC = false,
           bool WIDE = false>
-__global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
+__global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
+                                  fused_min_blocks<P, MIX, WIDE>())
     fused_colour_kernel(const DatasetDev *__restrict__ dsv,
                         ChainDev *__restrict__ chv,
                         const BlockMap *__restrict__ map, int colour,
                         Supplied sup) {
   static_assert(!TC || (!SUPP && !MIX && !WMU && LPV == 1),
                 "the tensor-core X'Z serves the probit production kernel");
-  static_assert(!WIDE || (!SUPP && !MIX && !TC && LPV == 1),
+  static_assert(!WIDE || MIX || (!SUPP && !TC && LPV == 1),
                 "the 16-subject step serves the probit production kernels");
   constexpr int NT = P * (P + 1) / 2;
   constexpr int PP = P <= 4 ? 4 : 8;  // design row padded to float4s
@@ -77,9 +79,13 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
   // other kernels keep one padded row per subject (a pad row per 32).
   constexpr bool PAIRX = !MIX && !SUPP;
   constexpr int RW = 2 * ((P + 1) & ~1);  // floats per pair row
-  // subjects staged per pass: half a chunk for the t/logit links, whose two
-  // tables of Philox words would not fit 48 KB beside a whole one
-  constexpr int CH = MIX ? kChunk / 2 : kChunk;
+  // TAB: the Philox calls' common words in tables (below).  Not for the
+  // t/logit links above P = 5 in blocks of 256: with eight warps per SM their
+  // latency counts (10 % longer sweeps at P = 8).
+  constexpr bool TAB = !SUPP && !(MIX && P > 5 && !WIDE);
+  // subjects staged per pass: half a chunk for the t/logit links with tables,
+  // which would not fit 48 KB beside a whole one
+  constexpr int CH = MIX && TAB ? kChunk / 2 : kChunk;
   constexpr int XS_FLOATS = PAIRX ? (CH / 2) * RW + (CH / 32) * 4 : (CH + CH / 32) * PP;
   __shared__ __align__(16) float Xs[XS_FLOATS];
   // The words of the chunk's Philox calls that do not depend on the voxel
@@ -88,8 +94,8 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
   // heavy FMA pipe, which all products of the generator go through, is the
   // busiest of the probit kernel (63 %): with a quarter of its products gone
   // the sweep of N = 1000, P = 5 takes 0.517 ms instead of 0.531.
-  __shared__ uint4 Zq[SUPP ? 1 : CH / 4 + CH / 32];
-  __shared__ uint4 Pq[MIX ? CH / 2 + CH / 32 : 1];
+  __shared__ uint4 Zq[TAB ? CH / 4 + CH / 32 : 1];
+  __shared__ uint4 Pq[MIX && TAB ? CH / 2 + CH / 32 : 1];
   __shared__ float Om[P * P], Xtx[P * P];
 
   const BlockMap bm = map[blockIdx.x];
@@ -179,11 +185,11 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         }
       }
     }
-    if constexpr (!SUPP) {
+    if constexpr (TAB) {
       for (int t = tid; t < cp / 4; t += blockDim.x)
         Zq[t + (t >> 3)] = philox_q((uint32_t)((i0 >> 2) + t), sweep, cid | kTagZ, key);
     }
-    if constexpr (MIX) {
+    if constexpr (MIX && TAB) {
       for (int t = tid; t < cp / 2; t += blockDim.x)
         Pq[t + (t >> 4)] = philox_q((uint32_t)((i0 >> 1) + t), sweep, cid | kTagPhi, key);
     }
@@ -497,12 +503,16 @@ __global__ void __launch_bounds__(256, fused_min_blocks<P, MIX, WIDE>())
         const uint32_t i00 = (uint32_t)(i0 + (wl << 5));
         // the latent words of subjects 4c..4c+3 of this word; MIX: the gamma
         // variates of subjects 2c, 2c + 1 (normal, uniform each)
-        const uint4 *zq = &Zq[SUPP ? 0 : 9 * wl], *pq = &Pq[MIX ? 17 * wl : 0];
+        const uint4 *zq = &Zq[TAB ? 9 * wl : 0], *pq = &Pq[MIX && TAB ? 17 * wl : 0];
         auto zcall = [&](int c) -> uint4 {
-          return SUPP ? make_uint4(0, 0, 0, 0) : philox_qv(zq[c], vlane, key);
+          if constexpr (SUPP) return make_uint4(0, 0, 0, 0);
+          if constexpr (TAB) return philox_qv(zq[c], vlane, key);
+          return philox(make_uint4((i00 >> 2) + c, (uint32_t)v, sweep, cid | kTagZ), key);
         };
         auto gpair = [&](int c) -> uint4 {
-          return MIX ? philox_qv(pq[c], vlane, key) : make_uint4(0, 0, 0, 0);
+          if constexpr (!MIX) return make_uint4(0, 0, 0, 0);
+          if constexpr (TAB) return philox_qv(pq[c], vlane, key);
+          return philox(make_uint4((i00 >> 1) + c, (uint32_t)v, sweep, cid | kTagPhi), key);
         };
         // MIX: the weights phi of a group of four subjects are loaded one
         // group ahead (the stores of the current group may alias as far as

@@ -24,6 +24,7 @@ constexpr int kGammaMax = 64;   // Marsaglia-Tsang attempts per gamma draw
 constexpr int kPostThreads = 256;   // block shape of the allocation-free
 constexpr int kPostPerThread = 4;   // Omega pass (bsg_noalloc.cu)
 constexpr int kMaxThreads = 256;    // largest block of the colour kernel
+constexpr int kSmallBlock = 128;    // the other one chosen for a group
 constexpr int kPredThreads = 128;   // subjects per block of the predictive pass
 constexpr int kPredWarps = 8;       // subjects (one warp each) per finishing block
 constexpr int kF64Threads = 64;     // threads of an FP64-chain block

@@ -87,7 +87,9 @@ bsg_status bsg_add_dataset(bsg_ctx *ctx, const bsg_dataset_desc *desc,
 bsg_status bsg_add_chain(bsg_ctx *ctx, int32_t dataset_id,
                          const bsg_chain_desc *desc, int32_t *chain_id);
 /* Tile shape of the fused colour kernel: lanes per voxel (1, 2, 4, 8) and
- * threads per block (64, 128, 256); 0 keeps the current choice. */
+ * threads per block (64, 128, 256); 0 keeps the current choice.  Until a
+ * block size is set, each launch group takes 256 or, where that spreads a
+ * small grid more evenly over the SMs, 128 (the results are the same). */
 bsg_status bsg_set_tuning(bsg_ctx *ctx, int32_t lanes_per_voxel,
                           int32_t block_threads);
 bsg_status bsg_get_tuning(const bsg_ctx *ctx, int32_t *lanes_per_voxel,
@@ -108,7 +110,7 @@ bsg_status bsg_set_tensor_xz(bsg_ctx *ctx, int32_t enable);
  * calls per step at two resident blocks of 128 registers, 8 draws two at
  * three blocks of 80 (P <= 5).  0 (the default) chooses per P group: 16
  * when P > 5, when the group's chains average N >= 384 subjects per voxel,
- * or when its grid is at most two blocks per SM; else 8.  The variates and
+ * or when two blocks per SM take no more waves than three; else 8.  The variates and
  * the arithmetic are the same, so the results are identical bit for bit.
  * bsg_get_step_subjects gives the largest step the context's plan uses
  * (0 when no chain is probit FP32).  No counterpart in the reference. */

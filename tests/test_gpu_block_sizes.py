@@ -21,7 +21,7 @@ def _study(shape, N, P, seed):
     return mask, covar, data
 
 
-def _run(study, threads, wm, chains=2, sweeps=3):
+def _run(study, threads, wm, chains=2, sweeps=3, model=None):
     import bsglmm_gb300 as bsg
     mask, covar, data = study
     w = np.random.default_rng(3).random(int(mask.sum())).astype(np.float32)
@@ -32,7 +32,10 @@ def _run(study, threads, wm, chains=2, sweeps=3):
         for c in ids:
             if wm:
                 s.set_wm_update(c, True)
-        s.set_tuning(1, threads)
+            if model:
+                s.set_model(c, model)
+        if threads:
+            s.set_tuning(1, threads)
         s.run(sweeps)
         for c in ids:
             out += [s.beta(c), s.omega(c), s.colmeans(c), *s.posterior(c)[:3], s.beta_wm(c)]
@@ -51,4 +54,18 @@ def test_block_sizes_agree_bit_for_bit(shape, N, P, wm):
     want = _run(study, 256, wm)
     for threads in (64, 128):
         for a, b in zip(_run(study, threads, wm), want):
+            assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("N,P,wm,model", [
+    (170, 3, False, None), (170, 5, True, None),
+    (40, 3, False, "logistic"), (40, 6, False, "t"), (33, 8, False, "logistic"),
+])
+def test_block_size_of_a_small_grid_gives_the_same_chain(N, P, wm, model):
+    """Few voxels and many subjects: blocks of 128 by default (above P = 5 the
+    t/logit kernel's form for them), against 256 and 64 set."""
+    study = _study((18, 17, 16), N, P, 40 + P)
+    want = _run(study, 0, wm, model=model)
+    for threads in (64, 256):
+        for a, b in zip(_run(study, threads, wm, model=model), want):
             assert np.array_equal(a, b)
