@@ -61,7 +61,7 @@ struct Group {
     int S = 0;
     std::vector<BlockMap> pmap, fmap;
     BlockMap *d_pmap = nullptr, *d_fmap = nullptr;
-    int pchunks = 0;
+    int pn = 0;  // most subjects of a chain
   };
   std::vector<Pred> pred;
 };
@@ -430,7 +430,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
         pr->pmap.push_back({(int32_t)ci, (int32_t)t, dsi, 0});
       for (int b = 0; b * kPredWarps < d.N; ++b)
         pr->fmap.push_back({(int32_t)ci, (int32_t)b, dsi, 0});
-      pr->pchunks = std::max(pr->pchunks, (d.N + kPredThreads - 1) / kPredThreads);
+      pr->pn = std::max(pr->pn, d.N);
     }
   }
   int nsm = 0;
@@ -518,15 +518,19 @@ cudaError_t enqueue_group(bsg_ctx *ctx, const Group &g, cudaStream_t st) {
   cudaError_t e;
   for (int c = 0; c < 2; ++c) {
     // the colour-0 latent phase reads beta_WM, which the previous colour-1
-    // kernel draws when the update is on: no early start then
-    const bool pdl = ctx->pdl && g.early && !(c == 0 && g.wm_any) && !g.fp64;
+    // kernel draws when the update is on: no early start then, unless the
+    // predictive pass lies between them (its kernels start their successors
+    // only after the wait that completes the colour-1 kernel)
+    const bool pdl =
+        ctx->pdl && g.early && !(c == 0 && g.wm_any && g.pred.empty()) && !g.fp64;
     e = launch_colour(ctx, g, c, st, pdl);
     if (e != cudaSuccess) return e;
   }
   for (const auto &pr : g.pred) {
     // DIC / Qhat pass; its blocks return at once unless the sweep is kept
-    e = launch_predict(g.P, pr.S, ctx->d_ds, ctx->d_ch, pr.d_pmap, (int)pr.pmap.size(),
-                       pr.pchunks, 0, kPredKept, st, ctx->pdl);
+    const int thr = pred_threads(pr.pn);
+    e = launch_predict(g.P, pr.S, ctx->d_ds, ctx->d_ch, pr.d_pmap, (int)pr.pmap.size(), thr,
+                       (pr.pn + thr - 1) / thr, 0, kPredKept, st, ctx->pdl);
     if (e != cudaSuccess) return e;
     e = launch_predict_finish(ctx->d_ds, ctx->d_ch, pr.d_fmap, (int)pr.fmap.size(), 0,
                               kPredKept, st, ctx->pdl);
@@ -599,13 +603,13 @@ bsg_status ensure_pred(bsg_ctx *ctx, Chain &c) {
   // Tiles sized so that one chain's grid (tiles x subject chunks) is about
   // one wave of resident blocks.
   const int ntot = (int)(d.vox[0].size() + d.vox[1].size());
-  const int chunks = (d.N + kPredThreads - 1) / kPredThreads;
+  const int threads = pred_threads(d.N), chunks = (d.N + threads - 1) / threads;
   int sms = 1;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  const int cap = sms * predict_blocks_per_sm(d.P, std::max(d.S, 1));
+  const int cap = sms * predict_blocks_per_sm(d.P, std::max(d.S, 1), threads);
   const int want = std::max(1, cap / std::max(chunks, 1));
   int tile = (ntot + want - 1) / want;
-  tile = std::max(kPredThreads, (tile + kPredThreads - 1) / kPredThreads * kPredThreads);
+  tile = std::max(kPredSub, (tile + kPredSub - 1) / kPredSub * kPredSub);
   const int T = std::max(1, (ntot + tile - 1) / tile);
   const size_t N = (size_t)d.N, G = (size_t)std::max(d.S, 1);
   cudaError_t e;
@@ -1822,8 +1826,8 @@ bsg_status bsg_predict(bsg_ctx *ctx, int32_t chain, double *mpredict) {
   bsg_status s = ensure_pred(ctx, c);
   if (s) return s;
   if ((s = build_plan(ctx))) return s;
-  const int chunks = (d.N + kPredThreads - 1) / kPredThreads;
-  CK(launch_predict(d.P, d.S, ctx->d_ds, ctx->d_ch, nullptr, c.dev.pred_tiles, chunks,
+  const int threads = pred_threads(d.N), chunks = (d.N + threads - 1) / threads;
+  CK(launch_predict(d.P, d.S, ctx->d_ds, ctx->d_ch, nullptr, c.dev.pred_tiles, threads, chunks,
                     chain, kPredNow, ctx->stream, false));
   CK(launch_predict_finish(ctx->d_ds, ctx->d_ch, nullptr,
                            (d.N + kPredWarps - 1) / kPredWarps, chain, kPredNow,
@@ -1868,8 +1872,8 @@ bsg_status bsg_get_dic(bsg_ctx *ctx, int32_t chain, double *dic) {
                 "DIC needs kept sweeps with the predictive pass on (bsg_set_predictive)");
   bsg_status s = build_plan(ctx);
   if (s) return s;
-  const int chunks = (d.N + kPredThreads - 1) / kPredThreads;
-  CK(launch_predict(d.P, d.S, ctx->d_ds, ctx->d_ch, nullptr, c.dev.pred_tiles, chunks,
+  const int threads = pred_threads(d.N), chunks = (d.N + threads - 1) / threads;
+  CK(launch_predict(d.P, d.S, ctx->d_ds, ctx->d_ch, nullptr, c.dev.pred_tiles, threads, chunks,
                     chain, kPredDE, ctx->stream, false));
   CK(launch_predict_finish(ctx->d_ds, ctx->d_ch, nullptr,
                            (d.N + kPredWarps - 1) / kPredWarps, chain, kPredDE,

@@ -25,8 +25,9 @@ constexpr int kPostThreads = 256;   // block shape of the allocation-free
 constexpr int kPostPerThread = 4;   // Omega pass (bsg_noalloc.cu)
 constexpr int kMaxThreads = 256;    // largest block of the colour kernel
 constexpr int kSmallBlock = 128;    // the other one chosen for a group
-constexpr int kPredThreads = 128;   // subjects per block of the predictive pass
-constexpr int kPredWarps = 8;       // subjects (one warp each) per finishing block
+constexpr int kPredMaxThreads = 256;  // most subjects per block of the predictive pass
+constexpr int kPredSub = 128;       // voxels it stages at a time
+constexpr int kPredWarps = 2;       // subjects (one warp each) per finishing block
 constexpr int kF64Threads = 64;     // threads of an FP64-chain block
 constexpr int kF64Lanes = 4;        // lanes per voxel of its small studies
 
@@ -117,7 +118,7 @@ struct ChainDev {
   int *any_status;         // the context's OR of every chain's bits
   // DIC / Qhat predictive pass (null until first used)
   int32_t pred_tiles;      // voxel tiles of the predictive pass
-  int32_t pred_tile;       // voxels per tile (a multiple of kPredThreads)
+  int32_t pred_tile;       // voxels per tile (a multiple of kPredSub)
   double *pred_part;       // [N][max(S,1)][tiles] per-tile subject sums
   double *pred_subj;       // [N] each subject's term of the ED / DE sum
   double *mpred;           // [N][S] Mpredict of the last pass
@@ -184,12 +185,20 @@ bool fused_supported(int P, int lpv, int threads);
 // Predictive pass (bsg_predict.cu).  With map == nullptr the grid is one
 // chain's tiles (blockIdx.x) or subject blocks; otherwise map[blockIdx.x]
 // holds {chain, tile} / {chain, subject block}.  chunks = subject blocks
-// of kPredThreads (gridDim.y).
+// of `threads` (gridDim.y; pred_threads).
 cudaError_t launch_predict(int P, int S, const DatasetDev *ds, ChainDev *ch,
-                           const BlockMap *map, int nblocks, int chunks, int chain,
-                           int mode, cudaStream_t st, bool pdl);
+                           const BlockMap *map, int nblocks, int threads, int chunks,
+                           int chain, int mode, cudaStream_t st, bool pdl);
 // Resident blocks per SM of predict_kernel<P, S>, for sizing its tiles.
-int predict_blocks_per_sm(int P, int S);
+int predict_blocks_per_sm(int P, int S, int threads);
+// Subjects (threads) per block for N subjects: the outcome words shared out
+// evenly over the fewest blocks of up to kPredMaxThreads (N = 403: 13 words as
+// 7 + 6, where blocks of 128 left three of sixteen warps without a subject).
+inline int pred_threads(int N) {
+  const int W = (N + 31) / 32, most = kPredMaxThreads / 32;
+  const int chunks = (W + most - 1) / most;
+  return 32 * ((W + chunks - 1) / chunks);
+}
 cudaError_t launch_predict_finish(const DatasetDev *ds, ChainDev *ch,
                                   const BlockMap *map, int nblocks, int chain,
                                   int mode, cudaStream_t st, bool pdl);

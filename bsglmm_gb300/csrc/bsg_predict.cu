@@ -10,7 +10,7 @@
 // reference launches 2 + S kernels and a blocking copy per subject; here one
 // launch covers every subject and voxel and a second reduces the tiles.
 //
-// predict_kernel<P, S>: a block takes 128 subjects (one per thread, the
+// predict_kernel<P, S>: a block takes up to 256 subjects (one per thread, the
 // design row in registers) and a tile of voxels, sized on the host so that
 // the grid is one wave, staged 128 at a time in shared memory (the voxel's
 // coefficients and beta_WM WM_v as float4s, and each warp's 32-subject
@@ -37,15 +37,13 @@ namespace bsg {
 
 namespace {
 
-constexpr int kPredSub = 128;  // voxels staged per pass (one per thread)
-// Resident blocks per SM asked of ptxas: 12 (40 registers, full occupancy;
-// measured faster than the 52-register schedule at 9 blocks) while the
-// design row and the group sums fit, fewer for larger P and S.
+// Resident blocks of 256 per SM asked of ptxas: 6 (40 registers, full
+// occupancy; measured faster than the 52-register schedule at three quarters
+// of it) while the design row and the group sums fit, fewer for larger P and S.
 template <int P, int S>
 constexpr int pred_min_blocks() {
-  return (P <= 5 && S <= 2) ? 12 : (P + S <= 8 ? 10 : 8);
+  return (P <= 5 && S <= 2) ? 6 : (P + S <= 8 ? 5 : 4);
 }
-static_assert(kPredSub == kPredThreads, "staging uses one voxel per thread");
 
 // A&S 26.2.17 with 1/sqrt(2 pi) folded in: c * (b1 t + ... + b5 t^5).
 constexpr float kA1 = 0.39894228f * 0.319381530f;
@@ -73,13 +71,14 @@ __device__ __forceinline__ float log2lik_as(float a) {
 __device__ __forceinline__ float2 log2lik_as2(float2 a) {
   const float2 h = fma2(splat2(0.2316419f), make_float2(fabsf(a.x), fabsf(a.y)), splat2(1.0f));
   const float2 t = make_float2(rcp_approx(h.x), rcp_approx(h.y));
-  const float2 r = mul2(t, fma2(t, fma2(t, fma2(t, fma2(t, splat2(kA5), splat2(kA4)),
-                                                splat2(kA3)), splat2(kA2)), splat2(kA1)));
+  // minus the polynomial, by its negated coefficients (the same bits but for
+  // the sign; f32x2 operands have no negation of their own)
+  const float2 r = mul2(t, fma2(t, fma2(t, fma2(t, fma2(t, splat2(-kA5), splat2(-kA4)),
+                                                splat2(-kA3)), splat2(-kA2)), splat2(-kA1)));
   const float2 w = mul2(mul2(a, splat2(-0.721347520f)), a);
-  const float2 fm = fma2(mul2(r, splat2(-1.f)),
-                         make_float2(ex2_approx(w.x), ex2_approx(w.y)), splat2(1.0f));
+  const float2 fm = fma2(r, make_float2(ex2_approx(w.x), ex2_approx(w.y)), splat2(1.0f));
   const bool t0 = a.x < 0.f, t1 = a.y < 0.f;
-  return add2(make_float2(lg2_approx(t0 ? r.x : fm.x), lg2_approx(t1 ? r.y : fm.y)),
+  return add2(make_float2(lg2_approx(t0 ? -r.x : fm.x), lg2_approx(t1 ? -r.y : fm.y)),
               make_float2(t0 ? w.x : 0.f, t1 ? w.y : 0.f));
 }
 
@@ -98,9 +97,10 @@ __device__ __forceinline__ float2 nlog2lik_logit2(float2 a) {
               make_float2(lg2_approx(e1.x), lg2_approx(e1.y)));
 }
 
-__device__ __forceinline__ float2 sign_flip2(float2 a, uint32_t m0, uint32_t m1) {
-  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ m0),
-                     __uint_as_float(__float_as_uint(a.y) ^ m1));
+// a with its signs flipped where the words' sign bits are clear (Y = 0)
+__device__ __forceinline__ float2 sign_flip2(float2 a, uint32_t y0, uint32_t y1) {
+  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ (~y0 & 0x80000000u)),
+                     __uint_as_float(__float_as_uint(a.y) ^ (~y1 & 0x80000000u)));
 }
 
 __device__ __forceinline__ bool predict_gate(const ChainDev &ch, int mode) {
@@ -114,7 +114,7 @@ __device__ __forceinline__ bool predict_gate(const ChainDev &ch, int mode) {
 // coefficients, then beta_WM WM_v), padded to float4s, so that each thread
 // evaluates two voxels per f32x2 operation.
 template <int P, int S>
-__global__ void __launch_bounds__(kPredThreads, pred_min_blocks<P, S>())
+__global__ void __launch_bounds__(kPredMaxThreads, pred_min_blocks<P, S>())
     predict_kernel(const DatasetDev *__restrict__ dsv, ChainDev *__restrict__ chv,
                    const BlockMap *__restrict__ map, int chain, int mode) {
   constexpr int R2 = (2 * (P + 1) + 3) / 4;  // float4s per staged voxel pair
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kPredThreads, pred_min_blocks<P, S>())
   const ChainDev &ch = chv[cidx];
   const DatasetDev &d = dsv[ch.dataset];
   const int N = d.N, Vp = d.Vp, V = d.V;
-  const int i0 = blockIdx.y * kPredThreads;
+  const int i0 = blockIdx.y * blockDim.x;
   if (i0 >= N || !predict_gate(ch, mode)) return;  // uniform per block
   const bool de = mode == kPredDE;
   const int n0 = d.n[0], ntot = n0 + d.n[1];
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kPredThreads, pred_min_blocks<P, S>())
   const int tw = ch.pred_tile;      // voxels per tile
 
   __shared__ float4 Bs2[kPredSub / 2][R2];
-  __shared__ uint32_t Ys[kPredThreads / 32][kPredSub];
+  __shared__ uint32_t Ys[kPredMaxThreads / 32][kPredSub];
 
   float2 xx[P];  // the subject's design row, duplicated for f32x2 operands
 #pragma unroll
@@ -159,11 +159,11 @@ __global__ void __launch_bounds__(kPredThreads, pred_min_blocks<P, S>())
   for (int q0 = t0; q0 < t1; q0 += kPredSub) {
     const int nsub = min(kPredSub, t1 - q0);
     __syncthreads();
-    if (tid < nsub) {
-      const int pos = q0 + tid;
+    for (int k = tid; k < nsub; k += blockDim.x) {
+      const int pos = q0 + k;
       const int c = pos < n0 ? 0 : 1, j = c ? pos - n0 : pos;
       const int sc = d.nb[c][j], v = d.vidx[c][j];
-      float *row = reinterpret_cast<float *>(&Bs2[tid >> 1][0]) + (tid & 1);
+      float *row = reinterpret_cast<float *>(&Bs2[k >> 1][0]) + (k & 1);
 #pragma unroll
       for (int p = 0; p < P; ++p)
         row[2 * p] = de ? (float)(ch.acc_sum[(size_t)p * V + v] * inv_nk)
@@ -198,8 +198,8 @@ __global__ void __launch_bounds__(kPredThreads, pred_min_blocks<P, S>())
             bp[2 * u + 1] = make_float2(f.z, f.w);
           }
           const uint2 yy = *reinterpret_cast<const uint2 *>(&Ys[warp][k]);
-          // sign masks: flip eta's sign when Y = 0
-          const uint32_t m0 = ~(yy.x << sh) & 0x80000000u, m1 = ~(yy.y << sh) & 0x80000000u;
+          // this subject's outcome in the sign bits: eta's flips when Y = 0
+          const uint32_t m0 = yy.x << sh, m1 = yy.y << sh;
           if (de) {
             float2 eta = bp[P];
 #pragma unroll
@@ -363,11 +363,11 @@ __global__ void __launch_bounds__(kPredWarps * 32)
 
 template <int P, int S>
 cudaError_t launch_predict_ps(const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
-                              int nblocks, int chunks, int chain, int mode,
+                              int nblocks, int threads, int chunks, int chain, int mode,
                               cudaStream_t st, bool pdl) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(nblocks, chunks);
-  cfg.blockDim = dim3(kPredThreads);
+  cfg.blockDim = dim3(threads);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -378,10 +378,10 @@ cudaError_t launch_predict_ps(const DatasetDev *ds, ChainDev *ch, const BlockMap
 }
 
 template <int P, int S>
-int predict_blocks_per_sm_ps() {
+int predict_blocks_per_sm_ps(int threads) {
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, predict_kernel<P, S>,
-                                                    kPredThreads, 0) != cudaSuccess)
+                                                    threads, 0) != cudaSuccess)
     return 1;
   return n > 0 ? n : 1;
 }
@@ -411,16 +411,17 @@ auto dispatch_ps(int P, int S, A... a) -> decltype(F<1, 1>::f(a...)) {
 template <int P, int S>
 struct LaunchF {
   static cudaError_t f(const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
-                       int nblocks, int chunks, int chain, int mode, cudaStream_t st,
-                       bool pdl) {
-    return launch_predict_ps<P, S>(ds, ch, map, nblocks, chunks, chain, mode, st, pdl);
+                       int nblocks, int threads, int chunks, int chain, int mode,
+                       cudaStream_t st, bool pdl) {
+    return launch_predict_ps<P, S>(ds, ch, map, nblocks, threads, chunks, chain, mode, st,
+                                   pdl);
   }
   static cudaError_t fail() { return cudaErrorInvalidValue; }
 };
 
 template <int P, int S>
 struct OccF {
-  static int f(int) { return predict_blocks_per_sm_ps<P, S>(); }
+  static int f(int threads) { return predict_blocks_per_sm_ps<P, S>(threads); }
   static int fail() { return 1; }
 };
 
@@ -462,13 +463,16 @@ __global__ void pairs_selftest_kernel(int64_t n, uint32_t k0, uint32_t k1,
 }  // namespace
 
 cudaError_t launch_predict(int P, int S, const DatasetDev *ds, ChainDev *ch,
-                           const BlockMap *map, int nblocks, int chunks, int chain,
-                           int mode, cudaStream_t st, bool pdl) {
+                           const BlockMap *map, int nblocks, int threads, int chunks,
+                           int chain, int mode, cudaStream_t st, bool pdl) {
   if (nblocks <= 0 || chunks <= 0) return cudaSuccess;
-  return dispatch_ps<LaunchF>(P, S, ds, ch, map, nblocks, chunks, chain, mode, st, pdl);
+  return dispatch_ps<LaunchF>(P, S, ds, ch, map, nblocks, threads, chunks, chain, mode, st,
+                              pdl);
 }
 
-int predict_blocks_per_sm(int P, int S) { return dispatch_ps<OccF>(P, S, 0); }
+int predict_blocks_per_sm(int P, int S, int threads) {
+  return dispatch_ps<OccF>(P, S, threads);
+}
 cudaError_t launch_predict_finish(const DatasetDev *ds, ChainDev *ch,
                                   const BlockMap *map, int nblocks, int chain,
                                   int mode, cudaStream_t st, bool pdl) {
