@@ -460,6 +460,11 @@ bsg_status build_plan(bsg_ctx *ctx) {
     const bool eligible = !g.mix && !g.fp64 && (g.wm_any || (ctx->lpv == 1 && !ctx->tc));
     g.wide = eligible && (ctx->step == 16 ||
                           (ctx->step == 0 && group_wide(g, blocks(kMaxThreads), nsm)));
+    // studies with the most subjects first: their blocks take longest, and a
+    // launch ends soonest when those do not start last
+    std::stable_sort(g.chains.begin(), g.chains.end(), [&](int x, int y) {
+      return ctx->ds[ctx->ch[x].dataset].N > ctx->ds[ctx->ch[y].dataset].N;
+    });
     for (int ci : g.chains)
       for (int c = 0; c < 2; ++c)
         map_chain(g.map[c], ci, ctx->ch[ci].dataset,
@@ -489,9 +494,6 @@ bsg_status build_plan(bsg_ctx *ctx) {
   return BSG_OK;
 }
 
-// Enqueues one sweep of every chain: per P group the two colour kernels
-// (groups on parallel branches when there are several); the colour-1
-// kernel also reduces the Omega pairs and draws Omega.
 // One colour kernel of a group.
 cudaError_t launch_colour(bsg_ctx *ctx, const Group &g, int c, cudaStream_t st, bool pdl) {
   if (g.fp64)
@@ -539,20 +541,24 @@ cudaError_t enqueue_group(bsg_ctx *ctx, const Group &g, cudaStream_t st) {
   return cudaSuccess;
 }
 
-cudaError_t enqueue_sweep(bsg_ctx *ctx, cudaStream_t st) {
-  cudaError_t e;
+// nsw sweeps of every chain: each group's on a branch of its own from the
+// first to the last (chains do not depend on one another), so that a sweep of
+// one group does not wait for the longest group's.
+cudaError_t enqueue_sweeps(bsg_ctx *ctx, cudaStream_t st, int64_t nsw) {
+  cudaError_t e = cudaSuccess;
   if (ctx->groups.size() == 1) {
-    if ((e = enqueue_group(ctx, ctx->groups[0], st)) != cudaSuccess) return e;
-  } else {
-    if ((e = cudaEventRecord(ctx->fork, st)) != cudaSuccess) return e;
-    for (size_t gi = 0; gi < ctx->groups.size(); ++gi) {
-      const Group &g = ctx->groups[gi];
-      cudaStream_t s = ctx->side[gi];
-      if ((e = cudaStreamWaitEvent(s, ctx->fork, 0)) != cudaSuccess) return e;
-      if ((e = enqueue_group(ctx, g, s)) != cudaSuccess) return e;
-      if ((e = cudaEventRecord(ctx->join[gi], s)) != cudaSuccess) return e;
-      if ((e = cudaStreamWaitEvent(st, ctx->join[gi], 0)) != cudaSuccess) return e;
-    }
+    for (int64_t i = 0; i < nsw && e == cudaSuccess; ++i)
+      e = enqueue_group(ctx, ctx->groups[0], st);
+    return e;
+  }
+  if ((e = cudaEventRecord(ctx->fork, st)) != cudaSuccess) return e;
+  for (size_t gi = 0; gi < ctx->groups.size(); ++gi) {
+    cudaStream_t s = ctx->side[gi];
+    if ((e = cudaStreamWaitEvent(s, ctx->fork, 0)) != cudaSuccess) return e;
+    for (int64_t i = 0; i < nsw; ++i)
+      if ((e = enqueue_group(ctx, ctx->groups[gi], s)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(ctx->join[gi], s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(st, ctx->join[gi], 0)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -565,8 +571,7 @@ bsg_status get_graph(bsg_ctx *ctx, int64_t nsw, cudaGraphExec_t *out) {
   }
   cudaGraph_t graph = nullptr;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = cudaSuccess;
-  for (int64_t s = 0; s < nsw && e == cudaSuccess; ++s) e = enqueue_sweep(ctx, ctx->stream);
+  cudaError_t e = enqueue_sweeps(ctx, ctx->stream, nsw);
   cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
   if (e != cudaSuccess || e2 != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
