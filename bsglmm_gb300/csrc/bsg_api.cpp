@@ -117,7 +117,7 @@ struct bsg_ctx {
 #endif
   std::map<int64_t, cudaGraphExec_t> graphs;
   void *pin = nullptr;  // pinned staging of bsg_step_host
-  size_t pin_bytes = 0;
+  void *pin_dev = nullptr;  // its device address
   bool pin_busy = false;  // copies through it may be in flight (a call ended early)
   std::string err;
 };
@@ -1088,47 +1088,36 @@ bsg_status bsg_step_host(bsg_ctx *ctx, int32_t chain, const double *omega_in,
   if (s) return s;
   const Chain &c = ctx->ch[chain];
   const int P = ctx->ds[c.dataset].P;
-  // staging: Omega in (FP64, FP32), Omega out, column means, status word
-  const size_t nd = sizeof(double) * P * P, nf = sizeof(float) * P * P;
-  const size_t need = 2 * nd + nf + sizeof(float) * P + sizeof(int);
-  if (ctx->pin_busy) {  // a previous call returned before its copies finished
+  // staging in pinned host memory, which the staging kernels address: Omega
+  // in, Omega out, column means, status word
+  const size_t nd = sizeof(double) * kMaxP * kMaxP;
+  const size_t need = 2 * nd + sizeof(float) * kMaxP + sizeof(int);
+  if (ctx->pin_busy) {  // a previous call returned before its staging finished
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->pin_busy = false;
   }
-  if (ctx->pin_bytes < need) {
-    if (ctx->pin) CK(cudaFreeHost(ctx->pin));
-    ctx->pin = nullptr;
-    ctx->pin_bytes = 0;
-    CK(cudaHostAlloc(&ctx->pin, need, cudaHostAllocDefault));
-    ctx->pin_bytes = need;
+  if (!ctx->pin) {
+    CK(cudaHostAlloc(&ctx->pin, need, cudaHostAllocMapped));
+    CK(cudaHostGetDevicePointer(&ctx->pin_dev, ctx->pin, 0));
   }
-  char *base = (char *)ctx->pin;
+  char *base = (char *)ctx->pin, *dev = (char *)ctx->pin_dev;
   double *in_d = (double *)base, *out_d = (double *)(base + nd);
-  float *in_f = (float *)(base + 2 * nd), *cm = (float *)(base + 2 * nd + nf);
-  int *bits = (int *)(base + 2 * nd + nf + sizeof(float) * P);
+  float *cm = (float *)(base + 2 * nd);
+  volatile int *bits = (int *)(base + 2 * nd + sizeof(float) * kMaxP);
   ctx->pin_busy = true;
   if (omega_in) {
-    for (int i = 0; i < P * P; ++i) {
-      in_d[i] = omega_in[i];
-      in_f[i] = (float)omega_in[i];
-    }
-    CK(cudaMemcpyAsync(c.dev.omega_d, in_d, nd, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(c.dev.omega_f, in_f, nf, cudaMemcpyHostToDevice, ctx->stream));
+    for (int i = 0; i < P * P; ++i) in_d[i] = omega_in[i];
+    CK(launch_stage_in((double *)dev, c.dev.omega_d, c.dev.omega_f, P * P, ctx->stream));
   }
   if (nsweeps > 0 && (s = bsg_run(ctx, nsweeps))) return s;
-  if (omega_out)
-    CK(cudaMemcpyAsync(out_d, c.dev.omega_d, nd, cudaMemcpyDeviceToHost, ctx->stream));
-  if (colmeans_out)
-    CK(cudaMemcpyAsync(cm, c.dev.colmean, sizeof(float) * P, cudaMemcpyDeviceToHost,
-                       ctx->stream));
   *bits = 0;
-  if (ctx->any_status)
-    CK(cudaMemcpyAsync(bits, ctx->any_status, sizeof(int), cudaMemcpyDeviceToHost,
-                       ctx->stream));
+  CK(launch_stage_out(c.dev.omega_d, c.dev.colmean, ctx->any_status, P, (double *)(dev + nd),
+                      (float *)(dev + 2 * nd), (int *)(dev + 2 * nd + sizeof(float) * kMaxP),
+                      ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->pin_busy = false;
   if (*bits) return bsg_sync(ctx);  // names the failing chains
-  if (omega_out) std::memcpy(omega_out, out_d, nd);
+  if (omega_out) std::memcpy(omega_out, out_d, sizeof(double) * P * P);
   if (colmeans_out) std::memcpy(colmeans_out, cm, sizeof(float) * P);
   return BSG_OK;
 }

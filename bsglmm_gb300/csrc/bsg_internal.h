@@ -181,6 +181,12 @@ cudaError_t launch_fill(float *p, size_t n, float value, cudaStream_t st);
 cudaError_t launch_pack(const uint8_t *bytes, int N, int V, int nc,
                         const int32_t *vidx, uint32_t *ybits, int *status,
                         cudaStream_t st);
+// The staging of a host-driven step (bsg_step_host): pinned host memory.
+cudaError_t launch_stage_in(const double *host, double *omega_d, float *omega_f, int n,
+                            cudaStream_t st);
+cudaError_t launch_stage_out(const double *omega_d, const float *colmean,
+                             const int *any_status, int P, double *out_d, float *cm,
+                             int *bits, cudaStream_t st);
 bool fused_supported(int P, int lpv, int threads);
 // Predictive pass (bsg_predict.cu).  With map == nullptr the grid is one
 // chain's tiles (blockIdx.x) or subject blocks; otherwise map[blockIdx.x]

@@ -94,6 +94,42 @@ cudaError_t launch_fill(float *p, size_t n, float value, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// ---------------------------------------------- host-driven steps (staging) --
+// Omega in from, and Omega, column means and the status word out to, a pinned
+// host buffer: one kernel each way.  Five small copies took about 20 us of a
+// step between them.
+__global__ void stage_in_kernel(const double *host, double *omega_d, float *omega_f, int n) {
+  const int i = threadIdx.x;
+  if (i < n) {
+    const double v = host[i];
+    omega_d[i] = v;
+    omega_f[i] = (float)v;
+  }
+}
+
+__global__ void stage_out_kernel(const double *omega_d, const float *colmean,
+                                 const int *any_status, int P, double *out_d, float *cm,
+                                 int *bits) {
+  const int i = threadIdx.x;
+  if (i < P * P) out_d[i] = omega_d[i];
+  if (i < P) cm[i] = colmean[i];
+  if (i == 0) *bits = *any_status;
+}
+
+cudaError_t launch_stage_in(const double *host, double *omega_d, float *omega_f, int n,
+                            cudaStream_t st) {
+  stage_in_kernel<<<1, kMaxP * kMaxP, 0, st>>>(host, omega_d, omega_f, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_stage_out(const double *omega_d, const float *colmean,
+                             const int *any_status, int P, double *out_d, float *cm,
+                             int *bits, cudaStream_t st) {
+  stage_out_kernel<<<1, kMaxP * kMaxP, 0, st>>>(omega_d, colmean, any_status, P, out_d, cm,
+                                               bits);
+  return cudaGetLastError();
+}
+
 // --------------------------------------------------- outcome bit packing --
 // data[i*V + v] bytes -> ybits[w*nc + j], bit b = subject 32w + b of the
 // voxel at colour position j.  Values other than 0/1 raise kErrInput.
