@@ -153,6 +153,12 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     vlane.init((uint32_t)v, sweep, key);
   }
   int ok = 1;
+  // (MIX: the link's constants are kept here: the stores of the weights may
+  // alias the chain's descriptor as far as the compiler knows)
+  const float t_df = MIX ? ch.t_df : 0.f, mix_d = MIX ? ch.mix_d : 0.f;
+  const float mix_c = MIX ? ch.mix_c : 0.f;
+  const uint32_t key0 = SUPP ? 0u : ch.key0, key1 = SUPP ? 0u : ch.key1;
+  float *const phv = MIX ? ch.phi[colour] + j : nullptr;  // this voxel's weights
   const uint32_t *yb = d.ybits[colour];
   // TC: the chunk's design slices and this warp's Z tile (dynamic shared
   // memory), the warp's four 8-voxel accumulator tiles, and whether any lane
@@ -222,7 +228,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
         if constexpr (MIX) {
           // standardised: (Z - mu) sqrt(phi) ~ N(0, 1) on (a, inf) after the
           // outcome's sign flip, a = -/+ mu sqrt(phi)
-          float *pp = ch.phi[colour] + (size_t)isub * nc + j;
+          float *pp = phv + (size_t)isub * nc;
           const float sd = rsqrt_approx(ph);
           const float a = __uint_as_float(__float_as_uint((m0 + bwm) * (ph * sd)) ^ ymask);
           float t = tn_lower_inv(fminf(a, kATail), kk);
@@ -232,17 +238,17 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           const float r = __uint_as_float(__float_as_uint(t * sd) ^ ymask ^ 0x80000000u);
           const float zr = m0 + r;  // Z - b_WM WM
           float gm;
-          if (ch.t_df == 3.f) {
+          if (t_df == 3.f) {
             // Gamma(2, 1) = Exp(1) + Exp(1) = -ln(u1 u2), exactly (t link)
             gm = __fmul_rn(lg2_approx(__fmul_rn(u_of(gn), u_of(gu))), -kLn2);
-          } else if (!gamma_mt_try(ch.mix_d, ch.mix_c, gn, gu, &gm)) {
-            gm = gamma_mt_more(ch.mix_d, ch.mix_c, isub, (uint32_t)v, sweep,
-                               cid | kTagPhiMore, ch.key0, ch.key1, &ok);
+          } else if (!gamma_mt_try(mix_d, mix_c, gn, gu, &gm)) {
+            gm = gamma_mt_more(mix_d, mix_c, isub, (uint32_t)v, sweep, cid | kTagPhiMore,
+                               key0, key1, &ok);
           }
           // the new weight 2 g / (r^2 + nu) with a MUFU reciprocal (r^2 + nu
           // >= 3; a few ulp, where the IEEE division's check and slow path
           // cost 4-6 % of the sweep)
-          const float phn = __fmul_rn(2.f * gm, rcp_approx(fmaf(r, r, ch.t_df)));
+          const float phn = __fmul_rn(2.f * gm, rcp_approx(fmaf(r, r, t_df)));
           *pp = phn;
           const float wz = phn * zr;
           float px[P];
@@ -400,7 +406,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
             if (P > 7) x[7] = v1.w;
           }
         };
-        const bool t3 = ch.t_df == 3.f;
+        const bool t3 = t_df == 3.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           float x[P];
@@ -438,7 +444,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           } else {
             float2 g;
             bool o0, o1;
-            gamma_mt_try2(ch.mix_d, ch.mix_c, gg.x, gg.z, gg.y, gg.w, &g, &o0, &o1);
+            gamma_mt_try2(mix_d, mix_c, gg.x, gg.z, gg.y, gg.w, &g, &o0, &o1);
             gq[q0] = g.x;
             gq[q1] = g.y;
             bad[q0] = !o0;
@@ -453,20 +459,20 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
             if (aq[q] > kATail) {
               const uint32_t ym = (yw4 >> q) << 31;
               const float t = tn_lower_tail(aq[q], i + q, (uint32_t)v, sweep,
-                                            cid | kTagZTail, ch.key0, ch.key1, &ok);
+                                            cid | kTagZTail, key0, key1, &ok);
               rq[q] = __uint_as_float(__float_as_uint(t * sdq[q]) ^ ym ^ 0x80000000u);
             }
             if (bad[q])
-              gq[q] = gamma_mt_more(ch.mix_d, ch.mix_c, i + q, (uint32_t)v, sweep,
-                                    cid | kTagPhiMore, ch.key0, ch.key1, &ok);
+              gq[q] = gamma_mt_more(mix_d, mix_c, i + q, (uint32_t)v, sweep,
+                                    cid | kTagPhiMore, key0, key1, &ok);
           }
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           float x[P];
           row(col0 + q, x);
-          const float phn = __fmul_rn(2.f * gq[q], rcp_approx(fmaf(rq[q], rq[q], ch.t_df)));
-          ch.phi[colour][(size_t)(i + q) * nc + j] = phn;
+          const float phn = __fmul_rn(2.f * gq[q], rcp_approx(fmaf(rq[q], rq[q], t_df)));
+          phv[(size_t)(i + q) * nc] = phn;
           const float wz = phn * (m0q[q] + rq[q]);
           float px[P];
 #pragma unroll
@@ -517,7 +523,6 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
         // MIX: the weights phi of a group of four subjects are loaded one
         // group ahead (the stores of the current group may alias as far as
         // the compiler knows, so it would not hoist them itself)
-        const float *phb = MIX ? ch.phi[colour] + j : nullptr;
         if constexpr (PAIRX) {
           // whole steps of kGroups calls, then (the end of a ragged last
           // word) steps of two calls or one, the last one perhaps reaching
@@ -557,14 +562,14 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           float phc[4] = {1.f, 1.f, 1.f, 1.f}, phx[4] = {1.f, 1.f, 1.f, 1.f};
           if (MIX) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) phc[q] = phb[(size_t)(i00 + q) * nc];
+            for (int q = 0; q < 4; ++q) phc[q] = phv[(size_t)(i00 + q) * nc];
           }
 #pragma unroll 1
           for (int b = 0; b < 32; b += 4) {
             const uint32_t i = i00 + (uint32_t)b;
             if (MIX && b + 4 < 32) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) phx[q] = phb[(size_t)(i + 4 + q) * nc];
+              for (int q = 0; q < 4; ++q) phx[q] = phv[(size_t)(i + 4 + q) * nc];
             }
             const uint4 r = zcall(b >> 2);
             if constexpr (MIX) {
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
               if (b + q < nbits)
                 subject(xo + b + q, yw << 31, variate(r, q, i + q), i + q,
                         (q & 1) ? gq.z : gq.x, (q & 1) ? gq.w : gq.y,
-                        MIX ? phb[(size_t)(i + q) * nc] : 1.f);
+                        MIX ? phv[(size_t)(i + q) * nc] : 1.f);
               yw >>= 1;
             }
           }
