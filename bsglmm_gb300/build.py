@@ -32,6 +32,8 @@ SOURCES = [
     "bsg_fp64.cu",
     "bsg_fused_tc.cu",
     "bsg_fused_wide.cu",
+    "bsg_fused_one.cu",
+    "bsg_fused_one_wide.cu",
     "bsg_kernels.cu",
     "bsg_peak.cu",
     "bsg_noalloc.cu",

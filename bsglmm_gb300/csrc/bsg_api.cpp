@@ -30,6 +30,7 @@ struct Dataset {
   std::vector<int32_t> idx, idxsc, vox[2];
   std::vector<uint8_t> nbrs[2];
   std::vector<int32_t> pad_of_v;  // padded index of compact mask index v
+  bool one = false;               // the first of several design columns is all ones
   DatasetDev dev{};               // device pointers
 };
 
@@ -51,6 +52,7 @@ struct Group {
   double vox = 0, subj_vox = 0;  // its chains' voxels and N x voxels
   int threads = 256;             // per block
   bool early = true;             // its kernels start early (programmatic launch)
+  bool one = false;              // first design column all ones (probit FP32 chains)
   std::vector<int> chains;
   std::vector<BlockMap> map[2];
   BlockMap *d_map[2] = {nullptr, nullptr};
@@ -401,9 +403,12 @@ bsg_status build_plan(bsg_ctx *ctx) {
     const bool mix = ctx->ch[ci].dev.model != 1;
     const bool wmu = ctx->ch[ci].dev.wm_update != 0;
     const int f64 = ctx->ch[ci].dev.fp64 ? f64_lanes(d) : 0;
+    const bool one = d.one && !mix && !f64;
     Group *g = nullptr;
     for (auto &gg : ctx->groups)
-      if (gg.P == d.P && gg.mix == mix && gg.wm_any == wmu && gg.fp64 == f64) g = &gg;
+      if (gg.P == d.P && gg.mix == mix && gg.wm_any == wmu && gg.fp64 == f64 &&
+          gg.one == one)
+        g = &gg;
     if (!g) {
       ctx->groups.push_back(Group());
       g = &ctx->groups.back();
@@ -411,6 +416,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
       g->mix = mix;
       g->wm_any = wmu;
       g->fp64 = f64;
+      g->one = one;
     }
     g->chains.push_back((int)ci);
     g->vox += (double)d.V;
@@ -502,6 +508,10 @@ cudaError_t launch_colour(bsg_ctx *ctx, const Group &g, int c, cudaStream_t st, 
   if (g.mix)
     return launch_fused_mix(g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
                             (int)g.map[c].size(), c, st, pdl);
+  if (g.one && (g.wm_any || (ctx->lpv == 1 && !ctx->tc)))
+    return (g.wide ? launch_fused_one_wide : launch_fused_one)(
+        g.P, g.threads, g.wm_any, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
+        st, pdl);
   if (g.wide)
     return launch_fused_wide(g.P, g.threads, g.wm_any, ctx->d_ds, ctx->d_ch, g.d_map[c],
                              (int)g.map[c].size(), c, st, pdl);
@@ -772,6 +782,8 @@ bsg_status bsg_add_dataset(bsg_ctx *ctx, const bsg_dataset_desc *desc,
   if (d.V == 0) return fail(ctx, BSG_ERR_INVALID, "mask is empty");
   if ((double)d.N * d.V > 4.0e12)
     return fail(ctx, BSG_ERR_UNSUPPORTED, "N*V too large");
+  d.one = d.P > 1;
+  for (int i = 0; i < d.N && d.one; ++i) d.one = q.covar[i] == 1.0f;
   // X'X in float, subject order (read_data.cpp:321-327).
   std::vector<float> xtx((size_t)d.P * d.P, 0.f);
   for (int i = 0; i < d.N; ++i)
@@ -1195,9 +1207,10 @@ int64_t bsg_launches_per_sweep(const bsg_ctx *ctx) {
   std::vector<int> ps, pp;
   for (auto &c : ctx->ch) {
     const Dataset &d = ctx->ds[c.dataset];
-    const int P = d.P * 8 + (c.dev.model != 1) * 2 + (c.dev.wm_update != 0) +
-                  (c.dev.fp64 ? 4 + (f64_lanes(d) > 1) : 0);
-    const int PS = d.P * 16 + d.S;
+    const int P = d.P * 16 + (c.dev.model != 1) * 2 + (c.dev.wm_update != 0) +
+                  (c.dev.fp64 ? 4 + (f64_lanes(d) > 1) : 0) +
+                  (d.one && c.dev.model == 1 && !c.dev.fp64 ? 8 : 0);
+    const int PS = P * 16 + d.S;
     if (std::find(ps.begin(), ps.end(), P) == ps.end()) ps.push_back(P);
     if (c.pred_on && std::find(pp.begin(), pp.end(), PS) == pp.end()) pp.push_back(PS);
   }

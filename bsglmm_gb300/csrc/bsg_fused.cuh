@@ -58,8 +58,15 @@ constexpr int fused_min_blocks() {
 // split product (bsg_mma.cuh), one lane per voxel; the rest is unchanged.
 // WIDE: the 16-subject whole-word step (identical results); for the t/logit
 // links above P = 5, the form for blocks of 128 threads.
+// ONE: studies whose first design column is all ones (an intercept): it is
+// not staged, x'beta starts from its coefficient and X'Z adds the draw itself,
+// which rounds as the products by one do, so the results are identical.  The
+// design's loads through the SM's one shared-memory path (40 bytes a lane and
+// subject pair at P = 5, 43 % of its time) fall by 1 / P; us per sweep with
+// and without, 230,285 voxels: N = 1000 P = 2 439 / 455, P = 5 503 / 516, P =
+// 8 566 / 577; N = 300 P = 3 152 / 158; 24 replicates 274 / 281.
 template <int P, int LPV, bool SUPP, bool MIX = false, bool WMU = false, bool TC = false,
-          bool WIDE = false>
+          bool WIDE = false, bool ONE = false>
 __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
                                   fused_min_blocks<P, MIX, WIDE>())
     fused_colour_kernel(const DatasetDev *__restrict__ dsv,
@@ -78,7 +85,10 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
   // a voxel (32 subjects = 16 pair rows apart) on distinct banks.  The
   // other kernels keep one padded row per subject (a pad row per 32).
   constexpr bool PAIRX = !MIX && !SUPP;
-  constexpr int RW = 2 * ((P + 1) & ~1);  // floats per pair row
+  static_assert(!ONE || (!SUPP && !MIX && !TC && LPV == 1 && P > 1),
+                "the intercept form serves the probit production kernels");
+  constexpr int P0 = ONE ? 1 : 0;  // first staged column
+  constexpr int RW = 2 * ((P - P0 + 1) & ~1);  // floats per pair row
   // TAB: the Philox calls' common words in tables (below).  Not for the
   // t/logit links above P = 5 in blocks of 256: with eight warps per SM their
   // latency counts (10 % longer sweeps at P = 8).
@@ -185,7 +195,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
         const float xv = ii < cn ? d.covar[(size_t)p * N + i0 + ii] : 0.f;
         if constexpr (PAIRX) {
           const int m = ii >> 1;
-          Xs[m * RW + (m >> 4) * 4 + 2 * p + (ii & 1)] = xv;
+          if (p >= P0) Xs[m * RW + (m >> 4) * 4 + 2 * (p - P0) + (ii & 1)] = xv;
         } else {
           Xs[(ii + (ii >> 5)) * PP + p] = xv;
         }
@@ -306,15 +316,15 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
 #pragma unroll
         for (int h = 0; h < H; ++h) {
           const float *xr = xr0 + h * RW;
-          float2 s = make_float2(0.f, 0.f);
+          float2 s = ONE ? bb[0] : make_float2(0.f, 0.f);
 #pragma unroll
-          for (int p = 0; p + 1 < P; p += 2) {
-            const float4 v4 = *reinterpret_cast<const float4 *>(xr + 2 * p);
+          for (int p = P0; p + 1 < P; p += 2) {
+            const float4 v4 = *reinterpret_cast<const float4 *>(xr + 2 * (p - P0));
             s = fma2(make_float2(v4.x, v4.y), bb[p], s);
             s = fma2(make_float2(v4.z, v4.w), bb[p + 1], s);
           }
-          if (P & 1)
-            s = fma2(*reinterpret_cast<const float2 *>(xr + 2 * (P - 1)), bb[P - 1], s);
+          if ((P - P0) & 1)
+            s = fma2(*reinterpret_cast<const float2 *>(xr + 2 * (P - 1 - P0)), bb[P - 1], s);
           m0h[h] = s;
           const float2 a = add2(s, make_float2(bwm, bwm));
           aq[2 * h] = __uint_as_float(__float_as_uint(a.x) ^ ((ywg >> (2 * h)) << 31));
@@ -365,7 +375,8 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
             const float z = (q & 1) ? zh[q >> 1].y : zh[q >> 1].x;
             if (i + q < (uint32_t)N) {
 #pragma unroll
-              for (int p = 0; p < P; ++p) acc2[p].x = fmaf(xr[2 * p], z, acc2[p].x);
+              for (int p = 0; p < P; ++p)
+                acc2[p].x = p < P0 ? acc2[p].x + z : fmaf(xr[2 * (p - P0)], z, acc2[p].x);
             }
           }
         } else {
@@ -373,14 +384,15 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           for (int h = 0; h < H; ++h) {
             const float *xr = xr0 + h * RW;
 #pragma unroll
-            for (int p = 0; p + 1 < P; p += 2) {
-              const float4 v4 = *reinterpret_cast<const float4 *>(xr + 2 * p);
+            for (int p = P0; p + 1 < P; p += 2) {
+              const float4 v4 = *reinterpret_cast<const float4 *>(xr + 2 * (p - P0));
               acc2[p] = fma2(make_float2(v4.x, v4.y), zh[h], acc2[p]);
               acc2[p + 1] = fma2(make_float2(v4.z, v4.w), zh[h], acc2[p + 1]);
             }
-            if (P & 1)
-              acc2[P - 1] = fma2(*reinterpret_cast<const float2 *>(xr + 2 * (P - 1)), zh[h],
+            if ((P - P0) & 1)
+              acc2[P - 1] = fma2(*reinterpret_cast<const float2 *>(xr + 2 * (P - 1 - P0)), zh[h],
                                  acc2[P - 1]);
+            if (ONE) acc2[0] = add2(acc2[0], zh[h]);
           }
         }
       };
@@ -1005,7 +1017,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
 // block of the previous kernel in the stream has passed its dependency
 // point.
 template <int P, int LPV, bool SUPP, bool MIX = false, bool WMU = false, bool TC = false,
-          bool WIDE = false>
+          bool WIDE = false, bool ONE = false>
 cudaError_t launch_one(int nblocks, int threads, cudaStream_t st, bool pdl,
                        const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
                        int colour, const Supplied &sup) {
@@ -1022,7 +1034,7 @@ cudaError_t launch_one(int nblocks, int threads, cudaStream_t st, bool pdl,
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, fused_colour_kernel<P, LPV, SUPP, MIX, WMU, TC, WIDE>, ds,
+  return cudaLaunchKernelEx(&cfg, fused_colour_kernel<P, LPV, SUPP, MIX, WMU, TC, WIDE, ONE>, ds,
                             ch, map, colour, sup);
 }
 

@@ -171,6 +171,15 @@ cudaError_t prepare_fused_tc();
 cudaError_t launch_fused_wide(int P, int threads, bool wmu, const DatasetDev *ds,
                               ChainDev *ch, const BlockMap *map, int nblocks, int colour,
                               cudaStream_t st, bool pdl);
+// The probit colour kernels of studies whose first design column is all ones
+// (P > 1; wmu: with the beta_WM update), one lane per voxel, Philox: 8- and
+// 16-subject steps (bsg_fused_one.cu, bsg_fused_one_wide.cu).
+cudaError_t launch_fused_one(int P, int threads, bool wmu, const DatasetDev *ds,
+                             ChainDev *ch, const BlockMap *map, int nblocks, int colour,
+                             cudaStream_t st, bool pdl);
+cudaError_t launch_fused_one_wide(int P, int threads, bool wmu, const DatasetDev *ds,
+                                  ChainDev *ch, const BlockMap *map, int nblocks, int colour,
+                                  cudaStream_t st, bool pdl);
 // The colour kernel of FP64 chains (bsg_fp64.cu): `lanes` (1 or kF64Lanes)
 // lanes per voxel, blocks of kF64Threads, Philox variates, probit link.
 cudaError_t launch_fp64(int P, int lanes, const DatasetDev *ds, ChainDev *ch,

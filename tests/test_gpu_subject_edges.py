@@ -36,6 +36,30 @@ def test_probit_sweep_matches_oracle(oracle_mod, N, step):
         assert np.allclose(s.beta(ch), o["beta"], rtol=TOL, atol=TOL)
 
 
+@pytest.mark.parametrize("P", [2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("step", [8, 16])
+@pytest.mark.parametrize("first", [True, False])
+def test_intercept_first_or_not_matches_oracle(oracle_mod, P, step, first):
+    """The form for a first design column of ones, and the general one (the
+    same design with its columns in the opposite order); with the beta_WM
+    update at even P."""
+    import bsglmm_gb300 as bsg
+    st = synth.small_study(600 + P, shape=(7, 6, 5), N=59, P=P, S=1)
+    covar = st.covar if first else np.ascontiguousarray(st.covar[::-1])
+    assert (covar[0] == 1).all() == first
+    wm = np.random.default_rng(P).random(st.V).astype(np.float32) if P % 2 == 0 else None
+    with bsg.Sampler() as s:
+        ds = s.add_dataset(st.mask, covar, st.data, 1, wm)
+        ch = s.add_chain(ds, seed=13, beta_wm=0.0 if wm is None else 0.3)
+        if wm is not None:
+            s.set_wm_update(ch, True)
+        s.set_step_subjects(step)
+        s.run(1)
+        pb = oracle_mod.Problem(st.mask, covar, st.data, 1, wm)
+        o = pb.chain(13, 1, beta_wm=0.0 if wm is None else 0.3, wm_update=wm is not None)
+        assert np.allclose(s.beta(ch), o["beta"], rtol=TOL, atol=TOL)
+
+
 @pytest.mark.parametrize("N", [1, 30, 32, 35, 511, 512, 513, 1030])
 def test_t_sweep_matches_oracle(oracle_mod, N):
     import bsglmm_gb300 as bsg
