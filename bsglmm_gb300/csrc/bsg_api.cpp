@@ -335,7 +335,9 @@ void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb)
 // P = 4: 38,456 voxels (151 blocks of 128) N = 60 25.7 / 29.4, N = 120 30.9 /
 // 33.2, N = 200 44.7 / 38.9, N = 350 73.4 / 55.6; 20,672 voxels N = 120 29.9 /
 // 28.9; 84,368 (165 blocks of 256) N = 120 48.6 / 51.2, N = 200 73.8 / 61.2;
-// 40,008 (157 blocks of 128, two on five SMs) N = 350 73.6 / 74.4.  The t and
+// 40,008 (157 blocks of 128, two on five SMs) N = 350 73.6 / 74.4.  Chains of
+// 1,556 voxels a colour (7 blocks of 256, 13 of 128), N = 50: 64 of them 43.4 /
+// 38.9, 128 79.9 / 74.4; 24 studies of up to 30,000 269 / 278.  The t and
 // logistic links (two lanes per voxel) cost three to four times as much a
 // subject: 8,552 voxels N = 60 50.2 / 46.6, 40,008 voxels N = 301 188 / 164.
 // The sums combine in one order, so the results do not depend on it.
@@ -345,6 +347,9 @@ int group_threads(const Group &g, int64_t b256, int64_t b128, int nsm, int threa
   // P > 5 t/logit: three blocks of 128 threads fit an SM, or one of 256 (with
   // more registers a thread); the latter is better where it fills each SM once
   if (g.mix && g.P > 5) return w256 <= 8 && w128 >= 8 ? kMaxThreads : kSmallBlock;
+  // many small studies: the smaller blocks' last ones have fewer idle threads
+  if (!g.mix && g.chains.size() > 1 && (double)b256 * 256 >= 1.05 * ((double)b128 * 128))
+    return kSmallBlock;
   if (w256 > 16 || w128 >= w256) return kMaxThreads;
   const double least = g.mix ? 32.0 : w256 <= 8 ? 150.0 : 160.0;
   return g.subj_vox >= least * g.vox ? kSmallBlock : kMaxThreads;
@@ -358,9 +363,10 @@ int group_threads(const Group &g, int64_t b256, int64_t b128, int nsm, int threa
 // 5 6.5 % less; 290,369 voxels (567 blocks) N = 50 90 / 81, N = 300 240 / 221;
 // N = 50, P = 3 chains of 7 blocks: 32 of them 33 / 29, 64 (448 blocks) 44 /
 // 55, 80 69 / 57, 128 81 / 91, 200 121 / 137.
-bool group_wide(const Group &g, int64_t b256, int nsm) {
+bool group_wide(const Group &g, int64_t blocks, int nsm) {
   constexpr int kWideMinN = 384;
-  const int64_t w2 = (b256 + 2 * nsm - 1) / (2 * nsm), w3 = (b256 + 3 * nsm - 1) / (3 * nsm);
+  const int64_t s2 = (int64_t)nsm * 2 * kMaxThreads / g.threads, s3 = s2 + s2 / 2;
+  const int64_t w2 = (blocks + s2 - 1) / s2, w3 = (blocks + s3 - 1) / s3;
   return g.P > 5 || g.subj_vox >= (double)kWideMinN * g.vox || w2 <= w3;
 }
 
@@ -465,7 +471,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
                 g.subj_vox >= 256.0 * g.vox);
     const bool eligible = !g.mix && !g.fp64 && (g.wm_any || (ctx->lpv == 1 && !ctx->tc));
     g.wide = eligible && (ctx->step == 16 ||
-                          (ctx->step == 0 && group_wide(g, blocks(kMaxThreads), nsm)));
+                          (ctx->step == 0 && group_wide(g, blocks(g.threads), nsm)));
     // studies with the most subjects first: their blocks take longest, and a
     // launch ends soonest when those do not start last
     std::stable_sort(g.chains.begin(), g.chains.end(), [&](int x, int y) {

@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kF64Threads)
     if (lane == 0) tot[q] = s;
   }
   __syncthreads();
-  if (warp == 0) wishart_warp(ch, d, tot, 0, Supplied{}, lane);
+  if (warp == 0) wishart_warp<P>(ch, tot, 0, Supplied{}, lane);
   if (warp == 1) sweep_end_warp(ch, d, tot, sweep_ll, kept, 0, lane);
 }
 

@@ -507,15 +507,16 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
       const int nw = (cn + 31) >> 5;
       // The outcome word is loaded one word ahead: taken where it is used, its
       // load stalled a warp 0.85 cycles per issue (0.49 now); sweep of N = 2000,
-      // P = 8 4 % shorter, of 1.5M voxels, N = 500 3.4 %.
+      // P = 8 4 % shorter, of 1.5M voxels, N = 500 3.4 %.  (The t/logit kernel
+      // has no register to spare for it: 0.5 to 1.6 % longer.)
       auto yload = [&](int wl) -> uint32_t {
         return (wl >= nw || (TC && !active)) ? 0u
                                              : __ldg(yb + (size_t)((i0 >> 5) + wl) * nc + j);
       };
       uint32_t ynext = yload(k);
       for (int wl = k; wl < nw; wl += LPV) {
-        uint32_t yw = ynext;
-        ynext = yload(wl + LPV);
+        uint32_t yw = MIX ? yload(wl) : ynext;
+        if (!MIX) ynext = yload(wl + LPV);
         const int nbits = min(32, cn - (wl << 5));
         const int xo = (wl << 5) + wl;  // padded offset of bit 0
         const uint32_t i00 = (uint32_t)(i0 + (wl << 5));
@@ -834,24 +835,6 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
       wmt = (double)wmv * (sz + (double)d.N * (double)bwm - sxb);
     }
 
-    // ---- posterior running sums of the kept sweep (mcmc.cpp:637-645): only
-    // this thread adds to these entries, by reductions at the L2 that it
-    // does not wait for (the same FP64 additions as a load, add and store)
-    if (kept) {
-#pragma unroll
-      for (int p = 0; p < P; ++p) {
-        const double x = (double)bnew[p];
-        atomicAdd(ch.acc_sum + (size_t)p * d.V + v, x);
-        atomicAdd(ch.acc_sq + (size_t)p * d.V + v, x * x);
-      }
-#pragma unroll
-      for (int g2 = 0; g2 < P; ++g2)
-        if (g2 < d.S)
-          atomicAdd(ch.prb_sum + (size_t)g2 * d.V + v,
-                    (double)(MIX ? prob_logit(bnew[g2], ch.inv_lf)
-                                 : prob_sdnorm(bnew[g2] + bwm)));
-    }
-
     // ---- Omega pair products (Spat_Coef_Prec, covarGPU.cu:953-1013) -----
     // Every in-mask edge joins a colour-0 and a colour-1 voxel, so the
     // colour-1 pass sees each edge once.  For a forward neighbour (+x, +y,
@@ -887,6 +870,29 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     atomicOr(ch.status, err);
     atomicOr(ch.any_status, err);
   }
+
+  // ---- posterior running sums of the kept sweep (mcmc.cpp:637-645): only
+  // this thread adds to these entries, by reductions at the L2 that it does
+  // not wait for (the same FP64 additions as a load, add and store); after the
+  // block's arrival, which waits for what the block has in flight (the t/logit
+  // kernel, whose end is short beside its draws, before it: up to 1 % better)
+  auto kept_sums = [&]() {
+    if (!leader || !kept) return;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const double x = (double)bnew[p];
+      atomicAdd(ch.acc_sum + (size_t)p * d.V + v, x);
+      atomicAdd(ch.acc_sq + (size_t)p * d.V + v, x * x);
+    }
+#pragma unroll
+    for (int g2 = 0; g2 < P; ++g2)
+      if (g2 < d.S)
+        atomicAdd(ch.prb_sum + (size_t)g2 * d.V + v,
+                  (double)(MIX ? prob_logit(bnew[g2], ch.inv_lf)
+                               : prob_sdnorm(bnew[g2] + bwm)));
+  };
+
+  if constexpr (MIX) kept_sums();
 
   // ---- block partials: column sums and the beta_WM term (both colours),
   // pairs (colour 1)
@@ -937,6 +943,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
       ch.partials0[(size_t)tid * ch.pstride0 + lb] = block_sum(tid < P ? kColOff + tid : kWmOff);
     // the last block to have read this colour's count advances it
     if (tid == 0 && arrived == (unsigned)(nblk - 1)) ch.sweep[0] = sweep_ll + 1;
+    if constexpr (!MIX) kept_sums();
     return;
   }
   if (tid < kFusedVals) {
@@ -951,7 +958,10 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     __threadfence();
   }
   __syncthreads();
-  if (!is_last) return;
+  if (!is_last) {
+    if constexpr (!MIX) kept_sums();
+    return;
+  }
   // Sums of the values over the blocks' rows (value-major) in a fixed order,
   // so the draw is bitwise reproducible: the rows of 256 threads' worth of
   // warps first (a tile, the same for every block size), then the tiles over
@@ -1008,8 +1018,9 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     if (lane % ln == 0 && mine < NV) tot[q] = s;
   }
   __syncthreads();
-  if (warp == 0) wishart_warp(ch, d, tot, SUPP ? 1 : 0, sup, lane);
+  if (warp == 0) wishart_warp<P>(ch, tot, SUPP ? 1 : 0, sup, lane);
   if (warp == 1) sweep_end_warp(ch, d, tot, sweep_ll, kept, SUPP ? 1 : 0, lane);
+  if constexpr (!MIX) kept_sums();
 }
 
 // Launch of one instantiation; with pdl the launch carries the

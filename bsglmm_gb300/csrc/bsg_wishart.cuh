@@ -80,110 +80,102 @@ static __device__ __forceinline__ double rsqrt_step(double d) {
 // the inverse is U^-T U^-1 and U^-T is lower triangular with a positive
 // diagonal, so chol((S + I)^-1) = U^-T (the Cholesky factor is unique),
 // and B = U^-T T comes from forward substitution without forming U^-T.
-static __device__ void wishart_warp(const ChainDev &ch, const DatasetDev &d,
-                                    const double *tot, int supplied,
+//
+// What counts is the depth of the chain, as nothing else of the sweep can go
+// on: lane q owns entry q of the packed lower triangle (P = 8: q + 32 too) in
+// registers, and P is a template argument, so that no index is computed at run
+// time (with run-time P and the matrices in shared memory it took 4.3 to 5.0 us
+// for P = 3; the sweep of the 20^3 study went from 19.7 to 17.8 us by this and
+// the kept sums' place after the block's arrival).
+template <int P>
+static __device__ void wishart_warp(const ChainDev &ch, const double *tot, int supplied,
                                     const Supplied &sup, int lane) {
-  __shared__ double A[kMaxP][kMaxP], T[kMaxP][kMaxP], B[kMaxP][kMaxP], rd[kMaxP];
-  const int P = d.P;
-  int err = 0;
-  // entry q of the packed lower triangle is (r, c), r >= c; the lanes take
-  // the entries (one round up to P = 7), so that every stage below is a
-  // few dependent FP64 operations deep (this part's FP64 pipe does two
-  // lanes per clock per SM, so depth, not width, sets the time)
-  auto rc_of = [](int q, int &r, int &c) {
-    r = 0;
-    while ((r + 1) * (r + 2) / 2 <= q) ++r;
-    c = q - r * (r + 1) / 2;
-  };
-  const int NP = P * (P + 1) / 2;
-  for (int q = lane; q < P * P; q += 32) {
-    const int r = q / P, c = q - r * P;
-    A[r][c] = (r >= c ? tot[tri(r, c)] : tot[tri(c, r)]) + (r == c ? 1.0 : 0.0);
-    T[r][c] = 0.0;
+  constexpr int NP = P * (P + 1) / 2, NE = (NP + 31) / 32;
+  __shared__ double U[P][P], B[P][P], piv;  // U[k][j]: U' by rows
+  int ei[NE], ej[NE];
+  double a[NE], t[NE];
+#pragma unroll
+  for (int u = 0; u < NE; ++u) {
+    const int q = lane + 32 * u;
+    int r = 0;
+#pragma unroll
+    for (int k = 1; k < P; ++k) r += q >= k * (k + 1) / 2;
+    ei[u] = q < NP ? r : -1;
+    ej[u] = q - r * (r + 1) / 2;
+    // S + I, and the Bartlett factor T: sqrt(chi^2) on the diagonal, normals
+    // below it (drawn by colour 1's last warp before its wait, or supplied)
+    a[u] = t[u] = 0.0;
+    if (q < NP) {
+      const bool dg = ei[u] == ej[u];
+      const int w = ei[u] * (ei[u] - 1) / 2 + ej[u];
+      a[u] = tot[q] + (dg ? 1.0 : 0.0);
+      t[u] = supplied ? (dg ? sqrt(sup.chi2[ei[u]]) : sup.wnorm[w])
+                      : __ldcg(ch.wdraw + (dg ? ei[u] : kMaxP + w));
+      if (q == NP - 1) piv = a[u];
+    }
   }
   __syncwarp();
-  // S + I = U U' with U upper, last pivot first; U goes to the upper
-  // triangle of A (diagonal included), the lower triangle holds the
-  // remaining leading block, rd[k] = 1 / U[k][k].
+  // S + I = U U' with U upper, last pivot first
   bool ok = true;
+  double rd[P];  // 1 / U[k][k]
+#pragma unroll
   for (int k = P - 1; k >= 0; --k) {
-    const double dk = A[k][k];
+    const double dk = piv;
     ok = ok && (dk > 0.0);
-    const double rs = rsqrt_step(dk);
+    rd[k] = rsqrt_step(dk);
+#pragma unroll
+    for (int u = 0; u < NE; ++u)
+      if (ei[u] == k) U[k][ej[u]] = a[u] * rd[k];
     __syncwarp();
-    if (lane < k) A[lane][k] = A[k][lane] * rs;
-    if (lane == k) {
-      A[k][k] = dk * rs;
-      rd[k] = rs;
-    }
-    __syncwarp();
-    for (int q = lane; q < k * (k + 1) / 2; q += 32) {
-      int i, j;
-      rc_of(q, i, j);
-      A[i][j] -= A[i][k] * A[j][k];
-    }
+#pragma unroll
+    for (int u = 0; u < NE; ++u)
+      if (ei[u] >= 0 && ei[u] < k) {
+        a[u] -= U[k][ei[u]] * U[k][ej[u]];
+        if (k > 0 && ei[u] == k - 1 && ej[u] == k - 1) piv = a[u];
+      }
     __syncwarp();
   }
+  int err = 0;
   if (ok) {
-    // T: the Bartlett factor, lower; sqrt(chi^2) on the diagonal and
-    // normals below it (drawn by the last colour-0 block of this sweep,
-    // or supplied)
-    const int nw = P * (P - 1) / 2;
-    if (lane < P) T[lane][lane] = supplied ? sqrt(sup.chi2[lane]) : __ldcg(ch.wdraw + lane);
-    if (lane < nw) {
-      int i = 1;
-      while ((i + 1) * i / 2 <= lane) ++i;  // row i: lane in [i(i-1)/2, i(i+1)/2)
-      const int j = lane - i * (i - 1) / 2;
-      T[i][j] = supplied ? sup.wnorm[lane] : __ldcg(ch.wdraw + kMaxP + lane);
-    }
-    __syncwarp();
-    // B = L T with L = U^-T, by forward substitution U' B = T (row i:
-    // B[i][.] = (T[i][.] - sum_{k<i} U[k][i] B[k][.]) / U[i][i]), right-
-    // looking so that each row costs two dependent FP64 operations; B is
-    // lower triangular like T
-    for (int q = lane; q < NP; q += 32) {
-      int i, j;
-      rc_of(q, i, j);
-      B[i][j] = T[i][j];
-    }
-    __syncwarp();
+    // B = U^-T T by forward substitution U' B = T, right-looking; B is lower
+    // triangular like T
+#pragma unroll
     for (int i = 0; i < P; ++i) {
-      if (lane <= i) B[i][lane] *= rd[i];
+#pragma unroll
+      for (int u = 0; u < NE; ++u)
+        if (ei[u] == i) B[i][ej[u]] = t[u] * rd[i];
       __syncwarp();
-      // rows r > i, columns j <= i: (P - 1 - i)(i + 1) <= 16 entries
-      const int nr = P - 1 - i;
-      if (lane < nr * (i + 1)) {
-        const int r = i + 1 + lane / (i + 1), j = lane - (lane / (i + 1)) * (i + 1);
-        B[r][j] -= A[i][r] * B[i][j];
-      }
-      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < NE; ++u)
+        if (ei[u] > i && ej[u] <= i) t[u] -= U[ei[u]][i] * B[i][ej[u]];
     }
-    __syncwarp();
     bool fin = true;
-    for (int q = lane; q < NP; q += 32) {  // Omega = B B', both triangles
-      int i, j;
-      rc_of(q, i, j);
-      double s = 0.0;
-      for (int k = 0; k <= j; ++k) s += B[i][k] * B[j][k];
-      A[i][j] = s;  // A is free again
-      A[j][i] = s;
-      fin = fin && isfinite(s);
+    double om[NE];
+#pragma unroll
+    for (int u = 0; u < NE; ++u) {  // Omega = B B'
+      om[u] = 0.0;
+      if (ei[u] >= 0) {
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+          if (k <= ej[u]) om[u] += B[ei[u]][k] * B[ej[u]][k];
+        fin = fin && isfinite(om[u]);
+      }
     }
     fin = __all_sync(0xffffffffu, fin);
-    __syncwarp();
     if (fin) {
-      for (int q = lane; q < P * P; q += 32) {
-        const int r = q / P, c = q - r * P;
-        ch.omega_d[q] = A[r][c];
-        ch.omega_f[q] = (float)A[r][c];
-      }
+#pragma unroll
+      for (int u = 0; u < NE; ++u)
+        if (ei[u] >= 0) {
+          const int lo = ei[u] * P + ej[u], up = ej[u] * P + ei[u];
+          ch.omega_d[lo] = ch.omega_d[up] = om[u];
+          ch.omega_f[lo] = ch.omega_f[up] = (float)om[u];
+        }
     } else {
       err |= kErrNaN;
     }
   } else {
     err |= kErrWishart;
   }
-  err = __reduce_or_sync(0xffffffffu, err);
   if (lane == 0 && err) {
     atomicOr(ch.status, err);
     atomicOr(ch.any_status, err);
