@@ -52,7 +52,7 @@ struct Group {
   double vox = 0, subj_vox = 0;  // its chains' voxels and N x voxels
   int threads = 256;             // per block
   bool early = true;             // its kernels start early (programmatic launch)
-  bool one = false;              // first design column all ones (probit FP32 chains)
+  bool one = false;              // first design column all ones (FP32 chains)
   std::vector<int> chains;
   std::vector<BlockMap> map[2];
   BlockMap *d_map[2] = {nullptr, nullptr};
@@ -276,10 +276,16 @@ int f64_lanes(const Dataset &d) {
   return std::max(d.vox[0].size(), d.vox[1].size()) < 38912 ? kF64Lanes : 1;
 }
 
+// Whether a chain runs the kernels for a first design column of ones.
+bool use_one(const Dataset &d, bool mix, bool f64) {
+  return d.one && !f64 && !(mix && d.P > 5);
+}
+
 // Partials of the colour kernels, one per block of a chain and value
 // (value-major, so that the last block's sums read consecutive blocks):
 // column sums (colour 0) and pairs + column sums (colour 1), sized for the
-// smallest tile the context launches; tot0 takes colour 0's totals.
+// smallest tile the chain can be launched in; tot0 takes an FP64 chain's
+// colour-0 totals, and the sweep's Bartlett variates behind them.
 bsg_status ensure_partials(bsg_ctx *ctx) {
   cudaError_t e;
   for (auto &c : ctx->ch) {
@@ -332,14 +338,20 @@ void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb)
 // the busiest SM fewer warps (grids of one wave: 77 blocks of 256 put eight
 // warps on half of the SMs, 152 of 128 four on each) and the subjects are
 // enough for that to count.  Measured, us per sweep with 256 / 128 threads,
-// P = 4: 38,456 voxels (151 blocks of 128) N = 60 25.7 / 29.4, N = 120 30.9 /
-// 33.2, N = 200 44.7 / 38.9, N = 350 73.4 / 55.6; 20,672 voxels N = 120 29.9 /
-// 28.9; 84,368 (165 blocks of 256) N = 120 48.6 / 51.2, N = 200 73.8 / 61.2;
-// 40,008 (157 blocks of 128, two on five SMs) N = 350 73.6 / 74.4.  Chains of
-// 1,556 voxels a colour (7 blocks of 256, 13 of 128), N = 50: 64 of them 43.4 /
-// 38.9, 128 79.9 / 74.4; 24 studies of up to 30,000 269 / 278.  The t and
-// logistic links (two lanes per voxel) cost three to four times as much a
-// subject: 8,552 voxels N = 60 50.2 / 46.6, 40,008 voxels N = 301 188 / 164.
+// P = 4 unless stated:
+//   8,552 voxels (34 blocks of 128)    N = 60 20.5 / 19.9, N = 120 28.2 / 22.9,
+//                                      N = 350 68.3 / 49.8
+//   15,000 (59)                        P = 5, N = 50 22.3 / 23.6
+//   38,456 (151)                       N = 60 23.4 / 26.3, N = 120 28.3 / 29.7,
+//                                      N = 200 42.2 / 35.5, N = 350 69.1 / 51.8
+//   40,008 (157, two on five SMs)      N = 350 73.6 / 74.4
+//   84,368 (330; 165 of 256)           N = 120 48.6 / 51.2, N = 200 73.8 / 61.2
+// and, several studies at once, for the idle threads of their last blocks:
+//   chains of 1,556 voxels a colour (7 blocks of 256, 13 of 128), P = 3, N =
+//   50: 64 of them 43.4 / 38.9, 128 79.9 / 74.4; 24 studies of up to 30,000
+//   voxels a colour 269 / 278.
+// The t and logistic links (two lanes per voxel) cost three to four times as
+// much a subject: 8,552 voxels N = 60 50.2 / 46.6, 40,008 N = 301 188 / 164.
 // The sums combine in one order, so the results do not depend on it.
 int group_threads(const Group &g, int64_t b256, int64_t b128, int nsm, int threads, bool set) {
   if (set || threads != kMaxThreads) return threads;
@@ -351,7 +363,7 @@ int group_threads(const Group &g, int64_t b256, int64_t b128, int nsm, int threa
   if (!g.mix && g.chains.size() > 1 && (double)b256 * 256 >= 1.05 * ((double)b128 * 128))
     return kSmallBlock;
   if (w256 > 16 || w128 >= w256) return kMaxThreads;
-  const double least = g.mix ? 32.0 : w256 <= 8 ? 150.0 : 160.0;
+  const double least = g.mix ? 32.0 : 4 * b128 <= nsm ? 40.0 : w256 <= 8 ? 150.0 : 160.0;
   return g.subj_vox >= least * g.vox ? kSmallBlock : kMaxThreads;
 }
 
@@ -409,7 +421,7 @@ bsg_status build_plan(bsg_ctx *ctx) {
     const bool mix = ctx->ch[ci].dev.model != 1;
     const bool wmu = ctx->ch[ci].dev.wm_update != 0;
     const int f64 = ctx->ch[ci].dev.fp64 ? f64_lanes(d) : 0;
-    const bool one = d.one && !mix && !f64;
+    const bool one = use_one(d, mix, f64 != 0);
     Group *g = nullptr;
     for (auto &gg : ctx->groups)
       if (gg.P == d.P && gg.mix == mix && gg.wm_any == wmu && gg.fp64 == f64 &&
@@ -512,8 +524,8 @@ cudaError_t launch_colour(bsg_ctx *ctx, const Group &g, int c, cudaStream_t st, 
     return launch_fp64(g.P, g.fp64, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
                        st);
   if (g.mix)
-    return launch_fused_mix(g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c],
-                            (int)g.map[c].size(), c, st, pdl);
+    return (g.one ? launch_fused_mix_one : launch_fused_mix)(
+        g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c, st, pdl);
   if (g.one && (g.wm_any || (ctx->lpv == 1 && !ctx->tc)))
     return (g.wide ? launch_fused_one_wide : launch_fused_one)(
         g.P, g.threads, g.wm_any, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
@@ -1222,7 +1234,7 @@ int64_t bsg_launches_per_sweep(const bsg_ctx *ctx) {
     const Dataset &d = ctx->ds[c.dataset];
     const int P = d.P * 16 + (c.dev.model != 1) * 2 + (c.dev.wm_update != 0) +
                   (c.dev.fp64 ? 4 + (f64_lanes(d) > 1) : 0) +
-                  (d.one && c.dev.model == 1 && !c.dev.fp64 ? 8 : 0);
+                  (use_one(d, c.dev.model != 1, c.dev.fp64 != 0) ? 8 : 0);
     const int PS = P * 16 + d.S;
     if (std::find(ps.begin(), ps.end(), P) == ps.end()) ps.push_back(P);
     if (c.pred_on && std::find(pp.begin(), pp.end(), PS) == pp.end()) pp.push_back(PS);

@@ -2,8 +2,8 @@
 // checkerboard colour it draws the Albert-Chib latent Z_iv for all
 // subjects from the packed outcome bits, accumulates X'(Z - b_WM WM) in
 // registers (Z never reaches memory), forms the conditional precision
-// Q = X'X + n_v Omega and mean vector, factors Q in registers and draws
-// beta_v.  With the new beta_v it also adds the kept sweep's FP64 running
+// Q = X'X + n_v Omega and mean vector, factors Q (once per block for each
+// n_v; per voxel for the t/logit links) and draws beta_v.  With the new beta_v it also adds the kept sweep's FP64 running
 // sums and the column sums, and (colour 1) the voxel's Omega pair products;
 // the last colour-1 block of a chain draws Omega.  A sweep is two launches.
 //
@@ -35,8 +35,8 @@ namespace bsg {
 // draws 8 from two calls at three blocks of 80 registers up to P = 5 (two
 // above).  On the brain-sized study (N = 1000, P = 5) WIDE is 6.5 % faster
 // per sweep; on 64 chains of a 50-subject study in one launch the narrow
-// form's extra resident warps win by 27 %.  BSG_FUSED_MIN_BLOCKS overrides
-// it for tuning builds.
+// form's extra resident warps win (38.9 us per sweep against 52.4).
+// BSG_FUSED_MIN_BLOCKS overrides it for tuning builds.
 template <int P, bool MIX = false, bool WIDE = false>
 constexpr int fused_min_blocks() {
 #ifdef BSG_FUSED_MIN_BLOCKS
@@ -78,16 +78,16 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
   static_assert(!WIDE || MIX || (!SUPP && !TC && LPV == 1),
                 "the 16-subject step serves the probit production kernels");
   constexpr int NT = P * (P + 1) / 2;
-  constexpr int PP = P <= 4 ? 4 : 8;  // design row padded to float4s
   // The probit kernel stages the design as subject pairs: pair row m holds
   // (x_2m,p, x_2m+1,p) for p = 0..P-1, so one f32x2 operation serves two
   // subjects; a pad of 4 floats after every 16 pair rows keeps the lanes of
   // a voxel (32 subjects = 16 pair rows apart) on distinct banks.  The
   // other kernels keep one padded row per subject (a pad row per 32).
   constexpr bool PAIRX = !MIX && !SUPP;
-  static_assert(!ONE || (!SUPP && !MIX && !TC && LPV == 1 && P > 1),
-                "the intercept form serves the probit production kernels");
+  static_assert(!ONE || (!SUPP && !TC && (MIX || LPV == 1) && P > 1),
+                "the intercept form serves the production kernels");
   constexpr int P0 = ONE ? 1 : 0;  // first staged column
+  constexpr int PP = P - P0 <= 4 ? 4 : 8;  // design row padded to float4s
   constexpr int RW = 2 * ((P - P0 + 1) & ~1);  // floats per pair row
   // TAB: the Philox calls' common words in tables (below).  Not for the
   // t/logit links above P = 5 in blocks of 256: with eight warps per SM their
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           const int m = ii >> 1;
           if (p >= P0) Xs[m * RW + (m >> 4) * 4 + 2 * (p - P0) + (ii & 1)] = xv;
         } else {
-          Xs[(ii + (ii >> 5)) * PP + p] = xv;
+          if (p >= P0) Xs[(ii + (ii >> 5)) * PP + p - P0] = xv;
         }
       }
     }
@@ -212,26 +212,25 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     if constexpr (TC) tc_stage_design<P>(tc_smem, d.covar, N, i0, cn, tid, blockDim.x);
     __syncthreads();
     if (run) {
+      // a subject's design row (not PAIRX; ONE: a 1 and the staged columns)
+      auto row = [&](int col, float (&x)[P]) {
+        float c[8];
+        const float4 v0 = *reinterpret_cast<const float4 *>(&Xs[col * PP]);
+        c[0] = v0.x, c[1] = v0.y, c[2] = v0.z, c[3] = v0.w;
+        if constexpr (PP == 8) {
+          const float4 v1 = *reinterpret_cast<const float4 *>(&Xs[col * PP + 4]);
+          c[4] = v1.x, c[5] = v1.y, c[6] = v1.z, c[7] = v1.w;
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) x[p] = p < P0 ? 1.f : c[p - P0];
+      };
       // One subject: mu = bwm + x'beta; a = -mu if Y = 1 else mu (sign-bit
       // flip by ymask = Y << 31); t ~ N(0,1) on (a, inf);
       // Z - bwm = x'beta + (Y ? t : -t); acc += x (Z - bwm).
       auto subject = [&](int col, uint32_t ymask, uint32_t kk, uint32_t isub,
                          uint32_t gn, uint32_t gu, float ph) {
         float x[P];
-        {
-          const float4 v0 = *reinterpret_cast<const float4 *>(&Xs[col * PP]);
-          x[0] = v0.x;
-          if (P > 1) x[1] = v0.y;
-          if (P > 2) x[2] = v0.z;
-          if (P > 3) x[3] = v0.w;
-          if (P > 4) {
-            const float4 v1 = *reinterpret_cast<const float4 *>(&Xs[col * PP + 4]);
-            x[4] = v1.x;
-            if (P > 5) x[5] = v1.y;
-            if (P > 6) x[6] = v1.z;
-            if (P > 7) x[7] = v1.w;
-          }
-        }
+        row(col, x);
         float m0 = 0.f;
 #pragma unroll
         for (int p = 0; p < P; ++p) m0 = fmaf(beta[p], x[p], m0);
@@ -404,20 +403,6 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
                             uint4 g1, const float (&ph4)[4]) {
         float m0q[4], aq[4], sdq[4], rq[4], gq[4];
         bool bad[4];
-        auto row = [&](int col, float (&x)[P]) {
-          const float4 v0 = *reinterpret_cast<const float4 *>(&Xs[col * PP]);
-          x[0] = v0.x;
-          if (P > 1) x[1] = v0.y;
-          if (P > 2) x[2] = v0.z;
-          if (P > 3) x[3] = v0.w;
-          if (P > 4) {
-            const float4 v1 = *reinterpret_cast<const float4 *>(&Xs[col * PP + 4]);
-            x[4] = v1.x;
-            if (P > 5) x[5] = v1.y;
-            if (P > 6) x[6] = v1.z;
-            if (P > 7) x[7] = v1.w;
-          }
-        };
         const bool t3 = t_df == 3.f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {

@@ -18,16 +18,16 @@ cudaError_t launch_mix(int nblocks, int threads, const DatasetDev *ds, ChainDev 
   const Supplied sup{};
   if constexpr (P > 5)
     if (threads <= kSmallBlock)
-      return launch_one<P, kMixLpv, false, true, false, false, true>(nblocks, threads, st, pdl,
-                                                                    ds, ch, map, colour, sup);
-  return launch_one<P, kMixLpv, false, true>(nblocks, threads, st, pdl, ds, ch, map, colour,
-                                             sup);
+      return launch_one<P, kMixLpv, false, true, false, false, true, false>(
+          nblocks, threads, st, pdl, ds, ch, map, colour, sup);
+  return launch_one<P, kMixLpv, false, true, false, false, false, false>(
+      nblocks, threads, st, pdl, ds, ch, map, colour, sup);
 }
 }  // namespace
 
 cudaError_t launch_fused_mix(int P, int threads, const DatasetDev *ds, ChainDev *ch,
-                             const BlockMap *map, int nblocks, int colour,
-                             cudaStream_t st, bool pdl) {
+                     const BlockMap *map, int nblocks, int colour, cudaStream_t st,
+                     bool pdl) {
   if (nblocks <= 0) return cudaSuccess;
   switch (P) {
     case 1: return launch_mix<1>(nblocks, threads, ds, ch, map, colour, st, pdl);

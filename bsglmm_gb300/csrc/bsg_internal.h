@@ -17,7 +17,6 @@ constexpr int kP0Vals = kMaxP + 1;
 constexpr int kFusedVals = kPostVals + 1;
 constexpr int kWmOff = kPostVals;                    // beta_WM term's slot
 constexpr int kChunk = 1024;                        // subjects staged per pass
-constexpr int kChunkPad = kChunk + kChunk / 32;     // one pad word per 32
 constexpr float kATail = 5.0f;  // inversion below, rejection above
 constexpr int kTailMax = 16;    // rejection attempts per latent draw
 constexpr int kGammaMax = 64;   // Marsaglia-Tsang attempts per gamma draw
@@ -107,7 +106,7 @@ struct ChainDev {
   double *partials1;       // [kFusedVals][pstride1] pairs, column sums, WM
                            // term of each colour-1 block (value-major)
   int32_t pstride0, pstride1;  // block rows allocated per value
-  double *tot0;            // [kP0Vals] colour-0 totals of the sweep
+  double *tot0;            // [kP0Vals] FP64 chains: colour-0 totals of the sweep
   double *wdraw;           // [kMaxP + kMaxPairs] the sweep's Bartlett variates:
                            // sqrt(chi^2) diagonal, then the normals
   unsigned int *done;      // [2] arrival counters of the colour kernels
@@ -159,6 +158,9 @@ constexpr int kMixLpv = 2;
 cudaError_t launch_fused_mix(int P, int threads, const DatasetDev *ds, ChainDev *ch,
                              const BlockMap *map, int nblocks, int colour,
                              cudaStream_t st, bool pdl);
+cudaError_t launch_fused_mix_one(int P, int threads, const DatasetDev *ds, ChainDev *ch,
+                                 const BlockMap *map, int nblocks, int colour,
+                                 cudaStream_t st, bool pdl);  // first column ones, P <= 5
 // The probit colour kernel with X'Z on the tensor cores (BF16x3 split, one
 // lane per voxel, Philox), bsg_fused_tc.cu.
 cudaError_t launch_fused_tc(int P, int threads, const DatasetDev *ds, ChainDev *ch,
