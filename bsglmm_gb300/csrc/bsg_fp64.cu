@@ -11,7 +11,7 @@
 //
 // What bounds it is the FP64 pipe (two lanes per clock and SM: a warp's
 // operation takes 16 cycles), so the latent draw is written for FP64
-// operations: about 63 + 2 P per subject and voxel.  CUDA's normcdf and
+// operations: about 55 + 2 P per subject and voxel.  CUDA's normcdf and
 // normcdfinv, which it used before, took some 330 and 2,120 instructions in
 // all, since the lanes of a warp go down both branches of each.
 #include "bsg_mills_table.h"
@@ -22,44 +22,48 @@ namespace {
 
 constexpr int kF64Chunk = 512;  // subjects of the design staged per pass
 constexpr int kF64Unroll = 2;   // subjects drawn side by side
+constexpr long long kATailBits = 0x4014000000000000ll;  // kATail = 5.0
+static_assert(kATail == 5.0f, "the bits above");
 
 // The tables of the draw, in shared memory (lanes index them apart).
 struct DrawTables {
   double mills[kMillsCoef][kMillsRows];
   double exp2[64];
+  double centre[kMillsRows];  // row / 8
 };
 
 __device__ void load_tables(DrawTables &tb, int tid, int nthreads) {
   for (int t = tid; t < kMillsRows * kMillsCoef; t += nthreads)
     tb.mills[t % kMillsCoef][t / kMillsCoef] = kMillsTable[t];
   for (int t = tid; t < 64; t += nthreads) tb.exp2[t] = kExp2Table[t];
+  for (int t = tid; t < kMillsRows; t += nthreads) tb.centre[t] = 0.125 * t;
 }
 
-// Mills ratio (1 - Phi(x)) / phi(x) for x >= 0: the row of the nearest
-// multiple of 1/8, found by adding 1.5 * 2^49 (whose last place is 1/8), and
-// a polynomial of degree 8 in the difference.  Beyond the table (x > 11.06)
-// the last row's centre: there Q(x) < 1e-28 only ever meets u >= 2^-33.
-__device__ __forceinline__ double mills(double x, const DrawTables &tb) {
-  const double m = x + 0x1.8p49;
-  const uint32_t j = (uint32_t)__double2loint(m);
-  double h = x - (m - 0x1.8p49);
-  if (j >= (uint32_t)kMillsRows) h = 0.0;
-  const uint32_t r = min(j, (uint32_t)kMillsRows - 1u);
-  double c = tb.mills[kMillsCoef - 1][r];
+// Mills ratio (1 - Phi(x)) / phi(x) for x = row / 8 + h, |h| <= 1/16 (and a
+// little over: rows are picked in FP32).
+__device__ __forceinline__ double mills(uint32_t row, double h, const DrawTables &tb) {
+  double c = tb.mills[kMillsCoef - 1][row];
 #pragma unroll
-  for (int i = kMillsCoef - 2; i >= 0; --i) c = fma(c, h, tb.mills[i][r]);
+  for (int i = kMillsCoef - 2; i >= 0; --i) c = fma(c, h, tb.mills[i][row]);
   return c;
 }
 
-// exp(y) for y <= 700 by a table of 2^(j/64) and a polynomial of degree 5
-// (Tang 1989); below -700 it stays at exp(-700).  n log(2)/64 is exact in its
-// leading part for the |n| < 2^17 that occur.
-__device__ __forceinline__ double exp_tab(double y, const DrawTables &tb) {
+// The row of x: the nearest multiple of 1/8.  Beyond the table (x > 11.06) the
+// last one, with h = 0: there Q(x) < 1e-28 only ever meets u >= 2^-33.
+__device__ __forceinline__ uint32_t mills_row(float x) {
+  return min((uint32_t)__float2int_rn(x * 8.f), (uint32_t)kMillsRows - 1u);
+}
+constexpr float kMillsEnd = 11.0625f;
+
+// exp(y + dy) for y <= 700 and a tiny dy (-0.0: none) by a table of 2^(j/64)
+// and a polynomial of degree 5 (Tang 1989); below -700 it stays at exp(-700).
+// n log(2)/64 is exact in its leading part for the |n| < 2^17 that occur.
+__device__ __forceinline__ double exp_tab(double y, double dy, const DrawTables &tb) {
   if ((uint32_t)__double2hiint(y) > 0xC085E000u) y = -700.0;
   const double m = fma(y, 9.23324826168936568e+01, 0x1.8p52);
   const int n = __double2loint(m);
   const double k = m - 0x1.8p52;
-  const double r = fma(k, -2.98158582698529328e-12, fma(k, -0x1.62e42fee00000p-7, y));
+  const double r = fma(k, -2.98158582698529328e-12, fma(k, -0x1.62e42fee00000p-7, y)) + dy;
   double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
   q = fma(q, r, 1.0 / 6.0);
   q = fma(q, r, 0.5);
@@ -87,20 +91,25 @@ __device__ __forceinline__ double tn_lower_inv_d(double a, uint32_t k, const Dra
   // u = (k + 1/2) 2^-32 exactly, from the double 2^52 + k; so is 1 - u
   const double u = fma(__hiloint2double(0x43300000, (int)k), 0x1p-32, -0x1p20 + 0x1p-33);
   const double uc = 1.0 - u;
-  const bool neg = a < 0.0;
+  const bool neg = __double2hiint(a) < 0;
   const double ax = fabs(a);
   // FP32: which tail, and the starting point
-  const float fu = u_of(k), fuc = u_of(~k), fT = phi_tail((float)ax);
+  const float fa = (float)ax;
+  const float fu = u_of(k), fuc = u_of(~k), fT = phi_tail(fa);
   const float ftuc = __fmul_rn(fT, fuc), fq = fmaf(fT, fuc, fu);
   const bool lo = neg && fq < 0.5f;
   const float x0 = -ndtri_lower(lo ? fq : (neg ? __fsub_rn(fuc, ftuc) : ftuc));
   // T sqrt(2 pi) = R(|a|) exp(-a^2 / 2), a^2 with its rounding error
   const double a2 = ax * ax, a2l = fma(ax, ax, -a2);
-  const double T = mills(ax, tb) * (exp_tab(-0.5 * a2, tb) * fma(-0.5, a2l, 1.0));
+  const uint32_t ra = mills_row(fa);
+  const double ha = fa > kMillsEnd ? 0.0 : ax - tb.centre[ra];
+  const double T = mills(ra, ha, tb) * exp_tab(-0.5 * a2, -0.5 * a2l, tb);
   const double A = lo ? u : (neg ? uc : 0.0);
   const double p = fma(flip_sign_d(uc, neg && !lo), T, A * kSqrt2Pi);
-  const double x = (double)x0, xx = x * x;
-  const double F = fma(-p, exp_tab(0.5 * xx, tb), mills(x, tb));
+  const double x = (double)x0, xx = x * x;  // exact
+  const uint32_t rx = mills_row(x0);
+  const double hx = (double)(x0 > kMillsEnd ? 0.f : x0 - 0.125f * (float)rx);  // exact
+  const double F = fma(-p, exp_tab(0.5 * xx, -0.0, tb), mills(rx, hx, tb));
   double d = fma(F, fma(xx, 1.0 / 3.0, 1.0 / 6.0), 0.5 * x);
   d = fma(F, d, 1.0);
   return flip_sign_d(fma(F, d, x), lo);
@@ -232,12 +241,13 @@ __global__ void __launch_bounds__(kF64Threads)
           y[q] = (yw >> ((i + q) & 31)) & 1u;
           a[q] = flip_sign_d(mu[q], y[q]);
           t[q] = tn_lower_inv_d(a[q], pick4(r, h + q), tb);
-          far = far || a[q] > (double)kATail;
+          // a > kATail, ordered as integers (a NaN counts as far)
+          far = far || __double_as_longlong(a[q]) > kATailBits;
         }
         if (far) {
 #pragma unroll
           for (int q = 0; q < kF64Unroll; ++q)
-            if (a[q] > (double)kATail && ii + q < cn)
+            if (__double_as_longlong(a[q]) > kATailBits && ii + q < cn)
               t[q] = tn_lower_tail_d(a[q], (uint32_t)(i + q), (uint32_t)v, sweep,
                                      cid | kTagZTail, ch.key0, ch.key1, &ok);
         }
