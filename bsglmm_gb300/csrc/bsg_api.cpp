@@ -270,8 +270,8 @@ constexpr int kParityThreads = 128;  // tile of the supplied-variate sweep
 // than eight warps on an SM of a GB300 (152 x 8 x 32 voxels of a colour), one
 // above, where four would only idle three lanes of each coefficient draw.
 // By the study alone, so that a chain's sums do not depend on what else its
-// context holds.  Measured at 9,424 voxels a colour, N = 117, P = 4: 0.79 ms
-// per sweep with one lane, 0.48 ms with four.
+// context holds.  Measured at 9,424 voxels a colour, N = 117, P = 4: 0.69 ms
+// per sweep with one lane, 0.44 ms with four.
 int f64_lanes(const Dataset &d) {
   return std::max(d.vox[0].size(), d.vox[1].size()) < 38912 ? kF64Lanes : 1;
 }
