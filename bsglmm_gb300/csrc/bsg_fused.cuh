@@ -346,12 +346,17 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
         if (__any_sync(__activemask(), amax > kATail)) {
 #pragma unroll
           for (int q = 0; q < 2 * H; ++q)
-            if (aq[q] > kATail && i + q < (uint32_t)N) {
-              const uint32_t ym = (ywg >> q) << 31;
-              const float t = tn_lower_tail(aq[q], i + q, (uint32_t)v, sweep,
-                                            cid | kTagZTail, ch.key0, ch.key1, &ok);
-              const float m0 = (q & 1) ? m0h[q >> 1].y : m0h[q >> 1].x;
-              const float z = m0 + __uint_as_float(__float_as_uint(t) ^ ym ^ 0x80000000u);
+            // (TC takes the whole last word: beyond N, where x = 0, a draw of
+            // 0, as the inversion far beyond kATail is not finite)
+            if (aq[q] > kATail && (TC || i + q < (uint32_t)N)) {
+              float z = 0.f;
+              if (i + q < (uint32_t)N) {
+                const uint32_t ym = (ywg >> q) << 31;
+                const float t = tn_lower_tail(aq[q], i + q, (uint32_t)v, sweep,
+                                              cid | kTagZTail, ch.key0, ch.key1, &ok);
+                const float m0 = (q & 1) ? m0h[q >> 1].y : m0h[q >> 1].x;
+                z = m0 + __uint_as_float(__float_as_uint(t) ^ ym ^ 0x80000000u);
+              }
               if (q & 1)
                 zh[q >> 1].y = z;
               else
