@@ -23,7 +23,9 @@ namespace {
 constexpr int kF64Chunk = 512;  // subjects of the design staged per pass
 constexpr int kF64Unroll = 2;   // subjects drawn side by side
 constexpr long long kATailBits = 0x4014000000000000ll;  // kATail = 5.0
+constexpr int kATailHi = 0x40140000;                    // its high word
 static_assert(kATail == 5.0f, "the bits above");
+constexpr uint32_t kFarHi = 0xC0428000u;  // high word of -37.0
 
 // The tables of the draw, in shared memory (lanes index them apart).
 struct DrawTables {
@@ -55,11 +57,10 @@ __device__ __forceinline__ uint32_t mills_row(float x) {
 }
 constexpr float kMillsEnd = 11.0625f;
 
-// exp(y + dy) for y <= 700 and a tiny dy (-0.0: none) by a table of 2^(j/64)
-// and a polynomial of degree 5 (Tang 1989); below -700 it stays at exp(-700).
-// n log(2)/64 is exact in its leading part for the |n| < 2^17 that occur.
+// exp(y + dy) for |y| <= 700 and a tiny dy (-0.0: none) by a table of 2^(j/64)
+// and a polynomial of degree 5 (Tang 1989).  n log(2)/64 is exact in its
+// leading part for the |n| < 2^17 that occur.
 __device__ __forceinline__ double exp_tab(double y, double dy, const DrawTables &tb) {
-  if ((uint32_t)__double2hiint(y) > 0xC085E000u) y = -700.0;
   const double m = fma(y, 9.23324826168936568e+01, 0x1.8p52);
   const int n = __double2loint(m);
   const double k = m - 0x1.8p52;
@@ -77,7 +78,8 @@ __device__ __forceinline__ double flip_sign_d(double x, bool flip) {
   return __hiloint2double(__double2hiint(x) ^ (flip ? (int)0x80000000 : 0), __double2loint(x));
 }
 
-// N(0,1) truncated to (a, +inf), a <= kATail, by inversion of u(k) in FP64:
+// N(0,1) truncated to (a, +inf), -37 < a <= kATail (beyond, what it returns is
+// replaced), by inversion of u(k) in FP64:
 // t = Phi^-1(Phi(a) + u Q(a)).  With T = Q(|a|) the upper tail of t is
 // p = T (1 - u) for a >= 0 and (1 - u) - T (1 - u) for a < 0; there, where
 // the lower tail p = u + T (1 - u) is below 1/2, it is taken instead, so that
@@ -114,6 +116,10 @@ __device__ __forceinline__ double tn_lower_inv_d(double a, uint32_t k, const Dra
   d = fma(F, d, 1.0);
   return flip_sign_d(fma(F, d, x), lo);
 }
+
+// The same for a <= -37: 1 - Q(a) is below 1e-299 and only ever meets u >=
+// 2^-33, while a^2 / 2 would leave exp_tab's range.
+__device__ __noinline__ double tn_lower_far_d(uint32_t k) { return normal_of_d(k); }
 
 // a > kATail: the Robert (1995) exponential-proposal rejection of
 // tn_lower_tail in FP64, on the same counters and attempt order.
@@ -241,15 +247,20 @@ __global__ void __launch_bounds__(kF64Threads)
           y[q] = (yw >> ((i + q) & 31)) & 1u;
           a[q] = flip_sign_d(mu[q], y[q]);
           t[q] = tn_lower_inv_d(a[q], pick4(r, h + q), tb);
-          // a > kATail, ordered as integers (a NaN counts as far)
-          far = far || __double_as_longlong(a[q]) > kATailBits;
+          // a > kATail or a <= -37, by the high words (a NaN counts as far)
+          const int hi = __double2hiint(a[q]);
+          far = far || hi >= kATailHi || (uint32_t)hi >= kFarHi;
         }
         if (far) {
 #pragma unroll
-          for (int q = 0; q < kF64Unroll; ++q)
-            if (__double_as_longlong(a[q]) > kATailBits && ii + q < cn)
+          for (int q = 0; q < kF64Unroll; ++q) {
+            if (ii + q >= cn) continue;
+            if (__double_as_longlong(a[q]) > kATailBits)
               t[q] = tn_lower_tail_d(a[q], (uint32_t)(i + q), (uint32_t)v, sweep,
                                      cid | kTagZTail, ch.key0, ch.key1, &ok);
+            else if ((uint32_t)__double2hiint(a[q]) >= kFarHi)
+              t[q] = tn_lower_far_d(pick4(r, h + q));
+          }
         }
 #pragma unroll
         for (int q = 0; q < kF64Unroll; ++q) {

@@ -26,3 +26,21 @@ def test_tensor_xz_far_tail_in_a_ragged_last_word(oracle_mod, N):
     o = oracle_mod.Problem(st.mask, st.covar, st.data, 1).chain(9, 1, beta_wm=15.0)
     # the split product's 2^-16 of |z - beta_WM WM| < 17, twice over
     assert np.allclose(b, o["beta"], rtol=1e-4, atol=2 * 17 * 2.0 ** -16)
+
+
+@pytest.mark.parametrize("bwm", [-36.0, -37.5, -200.0, -1e6, -1e14, -1e20, -1e30])
+def test_fp64_far_from_the_outcome(oracle_mod, bwm):
+    """FP64 chains with a mean far beyond the table of the Mills ratio, on
+    the outcome's own side (|a| up to 1e30; the far side is the tail
+    sampler's): finite, and the oracle's sweep."""
+    import bsglmm_gb300 as bsg
+    st = synth.small_study(42, shape=(9, 8, 7), N=37, P=3, S=1)
+    with bsg.Sampler() as s:
+        ch = s.add_chain(s.add_dataset(st.mask, st.covar, st.data, 1), seed=9, beta_wm=bwm)
+        s.set_precision(ch, 64)
+        s.run(1)
+        b = s.beta64(ch)
+    o = oracle_mod.Problem(st.mask, st.covar, st.data, 1).chain(9, 1, beta_wm=float(
+        np.float32(bwm)))
+    # FP64 on both sides: sums of N terms of up to |beta_WM|
+    assert np.allclose(b, o["beta"], rtol=1e-11, atol=1e-11 * (1.0 + abs(bwm)))
