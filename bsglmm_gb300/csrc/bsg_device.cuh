@@ -359,6 +359,18 @@ __device__ __forceinline__ float div_by(float x, float g, float r) {
   return fmaf(fmaf(-q, g, x), r, q);
 }
 
+// The reciprocals of a factor's diagonal.  An entry that is infinite (sums of
+// squares beyond a float) becomes 0 with reciprocal 0: quotients by it are 0
+// then as by division, where div_by's remainder would be a NaN.
+template <int P>
+__device__ __forceinline__ void diag_recip(float (&G)[P * (P + 1) / 2], float (&r)[P]) {
+#pragma unroll
+  for (int a = 0; a < P; ++a) {
+    r[a] = 1.f / G[tri(a, a)];
+    if (r[a] == 0.f) G[tri(a, a)] = 0.f;
+  }
+}
+
 template <int P>
 __device__ __forceinline__ void solve_lower(const float (&G)[P * (P + 1) / 2],
                                             const float (&r)[P], float (&x)[P]) {

@@ -346,21 +346,23 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
         if (__any_sync(__activemask(), amax > kATail)) {
 #pragma unroll
           for (int q = 0; q < 2 * H; ++q)
-            // (TC takes the whole last word: beyond N, where x = 0, a draw of
-            // 0, as the inversion far beyond kATail is not finite)
-            if (aq[q] > kATail && (TC || i + q < (uint32_t)N)) {
-              float z = 0.f;
-              if (i + q < (uint32_t)N) {
-                const uint32_t ym = (ywg >> q) << 31;
-                const float t = tn_lower_tail(aq[q], i + q, (uint32_t)v, sweep,
-                                              cid | kTagZTail, ch.key0, ch.key1, &ok);
-                const float m0 = (q & 1) ? m0h[q >> 1].y : m0h[q >> 1].x;
-                z = m0 + __uint_as_float(__float_as_uint(t) ^ ym ^ 0x80000000u);
-              }
+            if (aq[q] > kATail && i + q < (uint32_t)N) {
+              const uint32_t ym = (ywg >> q) << 31;
+              const float t = tn_lower_tail(aq[q], i + q, (uint32_t)v, sweep,
+                                            cid | kTagZTail, ch.key0, ch.key1, &ok);
+              const float m0 = (q & 1) ? m0h[q >> 1].y : m0h[q >> 1].x;
+              const float z = m0 + __uint_as_float(__float_as_uint(t) ^ ym ^ 0x80000000u);
               if (q & 1)
                 zh[q >> 1].y = z;
               else
                 zh[q >> 1].x = z;
+            } else if (TC && aq[q] > kATail) {
+              // (TC takes the whole last word: beyond N, where x = 0, a draw
+              // of 0, as the inversion far beyond kATail is not finite)
+              if (q & 1)
+                zh[q >> 1].y = 0.f;
+              else
+                zh[q >> 1].x = 0.f;
             }
         }
         if constexpr (TC) {
@@ -717,7 +719,10 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
 #pragma unroll
       for (int q = 0; q < NT; ++q) Gf[tid][q] = Q[q];
 #pragma unroll
-      for (int a = 0; a < P; ++a) Gf[tid][NT + a] = 1.f / Q[tri(a, a)];
+      for (int a = 0; a < P; ++a) {  // as diag_recip
+        Gf[tid][NT + a] = 1.f / Q[tri(a, a)];
+        if (Gf[tid][NT + a] == 0.f) Gf[tid][tri(a, a)] = 0.f;
+      }
     }
     __syncthreads();
   }
@@ -749,8 +754,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
         for (int q = 0; q <= a; ++q)
           Q[tri(a, q)] = qw[tri(a, q) < NQ ? tri(a, q) : 0] + (float)nnb * Om[q + a * P];
       okc = chol_packed<P>(Q);
-#pragma unroll
-      for (int a = 0; a < P; ++a) rd[a] = 1.f / Q[tri(a, a)];
+      diag_recip<P>(Q, rd);
     } else {
       okc = Gok[nnb];
 #pragma unroll

@@ -44,3 +44,28 @@ def test_fp64_far_from_the_outcome(oracle_mod, bwm):
         np.float32(bwm)))
     # FP64 on both sides: sums of N terms of up to |beta_WM|
     assert np.allclose(b, o["beta"], rtol=1e-11, atol=1e-11 * (1.0 + abs(bwm)))
+
+
+@pytest.mark.parametrize("model,P", [("probit", 2), ("probit", 6), ("t", 2), ("t", 7),
+                                     ("logistic", 3)])
+def test_squares_beyond_a_float(model, P):
+    """A first column of about 2e19: its sum of squares is infinite in FP32 and
+    its coefficient's conditional a spike at 0, as the division by its pivot
+    gives; the others' draws go on."""
+    import bsglmm_gb300 as bsg
+    rng = np.random.default_rng(4)
+    N, mask = 40, np.ones((6, 6, 6), np.uint8)
+    covar = rng.standard_normal((P, N)).astype(np.float32)
+    covar[0] *= 2e19
+    covar[-1] = 1
+    data = (rng.random((N, 216)) < 0.3).astype(np.uint8)
+    with bsg.Sampler() as s:
+        ch = s.add_chain(s.add_dataset(mask, covar, data, 1), seed=9)
+        s.set_model(ch, model)
+        s.run(1)
+        b = s.beta(ch)
+        s.run(3)
+        assert np.isfinite(s.beta(ch)).all() and not s.beta(ch)[0].any()
+    assert not b[0].any()
+    # bounded regression coefficients of a 0/1 outcome on unit-scale columns
+    assert np.abs(b[1:]).max() < 5 and (b[1:] != 0).any(axis=1).all()
