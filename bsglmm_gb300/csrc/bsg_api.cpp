@@ -339,19 +339,19 @@ void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb)
 // warps on half of the SMs, 152 of 128 four on each) and the subjects are
 // enough for that to count.  Measured, us per sweep with 256 / 128 threads,
 // P = 4 unless stated:
-//   8,552 voxels (34 blocks of 128)    N = 60 20.5 / 19.9, N = 120 28.2 / 22.9,
-//                                      N = 350 68.3 / 49.8
-//   15,000 (59)                        P = 5, N = 50 22.3 / 23.6
-//   38,456 (151)                       N = 60 23.4 / 26.3, N = 120 28.3 / 29.7,
-//                                      N = 200 42.2 / 35.5, N = 350 69.1 / 51.8
-//   40,008 (157, two on five SMs)      N = 350 73.6 / 74.4
-//   84,368 (330; 165 of 256)           N = 120 48.6 / 51.2, N = 200 73.8 / 61.2
+//   8,552 voxels (34 blocks of 128)    N = 60 20.4 / 19.2, N = 120 28.5 / 22.1,
+//                                      N = 350 69.2 / 50.1
+//   12,000 (47)                        P = 8, N = 50 28.6 / 29.3, N = 120 34.6 / 33.5
+//   38,456 (151)                       N = 50 21.8 / 22.7, N = 120 29.2 / 27.3,
+//                                      N = 200 42.9 / 33.4, N = 350 69.9 / 51.8
+//   40,008 (157, two on five SMs)      N = 350 69.9 / 70.5
+//   84,368 (330; 165 of 256)           N = 50 27.7 / 29.9, N = 120 46.9 / 42.3,
+//                                      N = 150 57.3 / 48.0, N = 200 71.2 / 58.8
 // and, several studies at once, for the idle threads of their last blocks:
 //   chains of 1,556 voxels a colour (7 blocks of 256, 13 of 128), P = 3, N =
-//   50: 64 of them 43.4 / 38.9, 128 79.9 / 74.4; 24 studies of up to 30,000
-//   voxels a colour 269 / 278.
+//   50: 64 of them 41.1 / 38.6, 128 76.8 / 71.1.
 // The t and logistic links (two lanes per voxel) cost three to four times as
-// much a subject: 8,552 voxels N = 60 50.2 / 46.6, 40,008 N = 301 188 / 164.
+// much a subject: 8,552 voxels N = 60 59.8 / 55.8, 40,008 N = 301 182 / 157.
 // The sums combine in one order, so the results do not depend on it.
 int group_threads(const Group &g, int64_t b256, int64_t b128, int nsm, int threads, bool set) {
   if (set || threads != kMaxThreads) return threads;

@@ -968,30 +968,49 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
   const int sub = kMaxThreads / blockDim.x;
   const int ntile = (nblk + sub - 1) / sub;
   const int nblk0 = max(1, (d.n[0] + vpb - 1) / vpb), ntile0 = (nblk0 + sub - 1) / sub;
-  auto tile = [&](const double *base, int nrow, int nt, int r) -> double {
+  // Tiles r, r + o, ... of a value, the loads of the first two rows of each in
+  // flight before any is used.  (Added as they came, blocks of 128 and 64 threads
+  // waited once for every tile; us per sweep at 450 tiles, N = 120, P = 4, before
+  // -> now: 128 threads 89 -> 78, 64 161 -> 132, 256 77 both.)
+  auto tiles = [&](auto &x, const double *base, int nrow, int r, int o) {
+    constexpr int T = sizeof(x) / sizeof(x[0]);
     auto ld = [&](int i) -> double { return i < nrow ? __ldcg(base + i) : 0.0; };
-    if (r >= nt) return 0.0;
-    if (sub == 1) return ld(r);
-    if (sub == 2) return ld(2 * r) + ld(2 * r + 1);
-    return (ld(4 * r) + ld(4 * r + 1)) + (ld(4 * r + 2) + ld(4 * r + 3));
+#pragma unroll
+    for (int u = 0; u < T; ++u) x[u] = ld(sub * (r + u * o));
+    if (sub > 1) {
+      double y[T];
+#pragma unroll
+      for (int u = 0; u < T; ++u) y[u] = ld(sub * (r + u * o) + 1);
+#pragma unroll
+      for (int u = 0; u < T; ++u) x[u] += y[u];
+    }
+    if (sub > 2) {
+      double y[T], z[T];
+#pragma unroll
+      for (int u = 0; u < T; ++u) {
+        y[u] = ld(sub * (r + u * o) + 2);
+        z[u] = ld(sub * (r + u * o) + 3);
+      }
+#pragma unroll
+      for (int u = 0; u < T; ++u) x[u] += y[u] + z[u];
+    }
   };
   const bool few = ntile <= 64;
   const int vw = few ? 4 : 1, ln = 32 / vw;  // values per warp, lanes per value
   auto rows = [&](const double *base, int nrow, int nt, double s) -> double {
     if (few) {
       for (int r = lane & 7; r < nt; r += 32) {
-        const double x0 = tile(base, nrow, nt, r), x1 = tile(base, nrow, nt, r + 8);
-        const double x2 = tile(base, nrow, nt, r + 16), x3 = tile(base, nrow, nt, r + 24);
-        s += x0;
-        if (r + 8 < nt) s += x1;
-        if (r + 16 < nt) s += x2;
-        if (r + 24 < nt) s += x3;
+        double x[4];
+        tiles(x, base, nrow, r, 8);
+        s += x[0];
+#pragma unroll
+        for (int u = 1; u < 4; ++u)
+          if (r + 8 * u < nt) s += x[u];
       }
     } else {
       for (int r = lane; r < nt; r += 256) {
         double x[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = tile(base, nrow, nt, r + 32 * u);
+        tiles(x, base, nrow, r, 32);
 #pragma unroll
         for (int w = 4; w > 0; w >>= 1)
 #pragma unroll
