@@ -360,14 +360,14 @@ __device__ __forceinline__ float div_by(float x, float g, float r) {
 }
 
 // The reciprocals of a factor's diagonal.  An entry that is infinite (sums of
-// squares beyond a float) becomes 0 with reciprocal 0: quotients by it are 0
-// then as by division, where div_by's remainder would be a NaN.
+// squares beyond a float) becomes the largest float, reciprocal 0: quotients by
+// it are 0 then as by division, where div_by's remainder would be a NaN.
 template <int P>
 __device__ __forceinline__ void diag_recip(float (&G)[P * (P + 1) / 2], float (&r)[P]) {
 #pragma unroll
   for (int a = 0; a < P; ++a) {
     r[a] = 1.f / G[tri(a, a)];
-    if (r[a] == 0.f) G[tri(a, a)] = 0.f;
+    G[tri(a, a)] = fminf(G[tri(a, a)], 3.402823466e38f);
   }
 }
 

@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
 #pragma unroll
       for (int q = 0; q < NT; ++q) Gf[tid][q] = Q[q];
 #pragma unroll
-      for (int a = 0; a < P; ++a) {  // as diag_recip
+      for (int a = 0; a < P; ++a) {  // as diag_recip (an infinite entry: 0)
         Gf[tid][NT + a] = 1.f / Q[tri(a, a)];
         if (Gf[tid][NT + a] == 0.f) Gf[tid][tri(a, a)] = 0.f;
       }
@@ -968,31 +968,48 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
   const int sub = kMaxThreads / blockDim.x;
   const int ntile = (nblk + sub - 1) / sub;
   const int nblk0 = max(1, (d.n[0] + vpb - 1) / vpb), ntile0 = (nblk0 + sub - 1) / sub;
-  // Tiles r, r + o, ... of a value, the loads of the first two rows of each in
-  // flight before any is used.  (Added as they came, blocks of 128 and 64 threads
-  // waited once for every tile; us per sweep at 450 tiles, N = 120, P = 4, before
-  // -> now: 128 threads 89 -> 78, 64 161 -> 132, 256 77 both.)
-  auto tiles = [&](auto &x, const double *base, int nrow, int r, int o) {
+  auto ld = [](const double *base, int nrow, int i) -> double {
+    return i < nrow ? __ldcg(base + i) : 0.0;
+  };
+  auto tile = [&](const double *base, int nrow, int nt, int r) -> double {
+    if (r >= nt) return 0.0;
+    if (sub == 1) return ld(base, nrow, r);
+    if (sub == 2) return ld(base, nrow, 2 * r) + ld(base, nrow, 2 * r + 1);
+    return (ld(base, nrow, 4 * r) + ld(base, nrow, 4 * r + 1)) +
+           (ld(base, nrow, 4 * r + 2) + ld(base, nrow, 4 * r + 3));
+  };
+  // Tiles r, r + o, ... of a value.  Their first two rows are loaded before any is
+  // used: added as they come (`tile`), blocks of 128 and 64 threads wait once for
+  // every tile; us per sweep at 450 tiles, N = 120, P = 4, as they come / ahead:
+  // 128 threads 89 / 78, 64 161 / 132, 256 77 both.  Not for the t/logit links up
+  // to P = 5, whose registers it costs 1 % of a sweep at P = 5 (P = 8, above: 1021
+  // / 912).
+  constexpr bool AHEAD = !(MIX && P <= 5);
+  auto tiles = [&](auto &x, const double *base, int nrow, int nt, int r, int o) {
     constexpr int T = sizeof(x) / sizeof(x[0]);
-    auto ld = [&](int i) -> double { return i < nrow ? __ldcg(base + i) : 0.0; };
+    if constexpr (!AHEAD) {
 #pragma unroll
-    for (int u = 0; u < T; ++u) x[u] = ld(sub * (r + u * o));
-    if (sub > 1) {
-      double y[T];
+      for (int u = 0; u < T; ++u) x[u] = tile(base, nrow, nt, r + u * o);
+    } else {
 #pragma unroll
-      for (int u = 0; u < T; ++u) y[u] = ld(sub * (r + u * o) + 1);
+      for (int u = 0; u < T; ++u) x[u] = ld(base, nrow, sub * (r + u * o));
+      if (sub > 1) {
+        double y[T];
 #pragma unroll
-      for (int u = 0; u < T; ++u) x[u] += y[u];
-    }
-    if (sub > 2) {
-      double y[T], z[T];
+        for (int u = 0; u < T; ++u) y[u] = ld(base, nrow, sub * (r + u * o) + 1);
 #pragma unroll
-      for (int u = 0; u < T; ++u) {
-        y[u] = ld(sub * (r + u * o) + 2);
-        z[u] = ld(sub * (r + u * o) + 3);
+        for (int u = 0; u < T; ++u) x[u] += y[u];
       }
+      if (sub > 2) {
+        double y[T], z[T];
 #pragma unroll
-      for (int u = 0; u < T; ++u) x[u] += y[u] + z[u];
+        for (int u = 0; u < T; ++u) {
+          y[u] = ld(base, nrow, sub * (r + u * o) + 2);
+          z[u] = ld(base, nrow, sub * (r + u * o) + 3);
+        }
+#pragma unroll
+        for (int u = 0; u < T; ++u) x[u] += y[u] + z[u];
+      }
     }
   };
   const bool few = ntile <= 64;
@@ -1001,7 +1018,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     if (few) {
       for (int r = lane & 7; r < nt; r += 32) {
         double x[4];
-        tiles(x, base, nrow, r, 8);
+        tiles(x, base, nrow, nt, r, 8);
         s += x[0];
 #pragma unroll
         for (int u = 1; u < 4; ++u)
@@ -1010,7 +1027,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     } else {
       for (int r = lane; r < nt; r += 256) {
         double x[8];
-        tiles(x, base, nrow, r, 32);
+        tiles(x, base, nrow, nt, r, 32);
 #pragma unroll
         for (int w = 4; w > 0; w >>= 1)
 #pragma unroll
