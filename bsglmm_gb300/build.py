@@ -35,6 +35,8 @@ SOURCES = [
     "bsg_fused_wide.cu",
     "bsg_fused_one.cu",
     "bsg_fused_one_wide.cu",
+    "bsg_fused_rel.cu",
+    "bsg_fused_rel_one.cu",
     "bsg_kernels.cu",
     "bsg_peak.cu",
     "bsg_noalloc.cu",

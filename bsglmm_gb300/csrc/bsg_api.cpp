@@ -51,7 +51,7 @@ struct Group {
   bool wide = false;    // the 16-subject whole-word step (bsg_fused_wide.cu)
   double vox = 0, subj_vox = 0;  // its chains' voxels and N x voxels
   int threads = 256;             // per block
-  bool early = true;             // its kernels start early (programmatic launch)
+  bool release = false;          // the next kernel let in within the subject loop
   bool one = false;              // first design column all ones (FP32 chains)
   std::vector<int> chains;
   std::vector<BlockMap> map[2];
@@ -328,10 +328,57 @@ bsg_status ensure_partials(bsg_ctx *ctx) {
 // alternating (a colour kernel's early phase reads its own colour's state,
 // final once the other colour's kernel has passed its dependency point),
 // so neither colour's launch may be left out.
-void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb) {
-  if (n == 0) m.push_back({(int32_t)chain, 0, (int32_t)dataset, 0});
+void map_chain(std::vector<BlockMap> &m, int chain, int dataset, int n, int vpb,
+               int release = -1) {
+  if (n == 0) m.push_back({(int32_t)chain, 0, (int32_t)dataset, (int32_t)release});
   for (int s = 0; s < n; s += vpb)
-    m.push_back({(int32_t)chain, (int32_t)s, (int32_t)dataset, 0});
+    m.push_back({(int32_t)chain, (int32_t)s, (int32_t)dataset, (int32_t)release});
+}
+
+// Whether a chain gains by letting the next kernel in within its subjects
+// (the place of the dependency protocol's wait) instead of after the last, on a
+// grid of up to one block per SM.  Let in after the last, the next kernel's
+// blocks are placed when some of this one's have left, two of them on an SM of
+// which others then have none; once that mode sets in it lasts.  Where the
+// subjects are few, the previous kernel's end (block sums, Omega draw) is not
+// over and the wait costs more than it gives.  A t/logit chain's ragged last
+// word, drawn one subject at a time, counts fourfold; from N = 64 to 80 the place
+// would be in the first word, too early; at P = 5 the check costs the t/logit
+// kernel's 128 registers 3 to 5 %.  us per sweep, after the last / within:
+//   75,000 voxels (147 blocks of 256)  P = 2, N = 120 34.6 / 24.6, N = 200 52 / 33.5,
+//                                      P = 4, N = 100 28.4 / 27.5, N = 200 57 / 39.4,
+//                                      P = 8, N = 200 53.8 / 54.1, N = 400 124 / 85
+//   6,000 (12 of 256, 24 of 128)       P = 2, N = 50 15.1 / 15.5, N = 120 20.2 / 18.5,
+//                                      P = 4, N = 100 21.3 / 21.2, N = 150 26.9 / 24.2,
+//                                      P = 8, N = 150 35.4 / 35.2, N = 400 69 / 54
+//   38,400 (150), t, P = 2             N = 25 37.2 / 25.6, N = 33 21.7 / 22.9, N = 64
+//                                      20.8 / 21.9, N = 120 66 / 44, N = 333 91 / 63
+//   the same, logistic                 P = 3, N = 333 146 / 100, P = 5, N = 64 34.1 /
+//                                      38.3, N = 128 38.5 / 40.1, N = 250 123 / 115
+bool gains_by_release(const Group &g, int N) {
+  if (!g.mix) return N >= 64 + 20 * g.P;
+  if (g.P == 5) return N >= 200;
+  return N > 80 || (N < 64 && N + 3 * (N % 32) >= 76);
+}
+
+// The group's kernels are of the form with that wait (REL).
+bool group_release(const bsg_ctx *ctx, const Group &g, int64_t blocks, int nsm) {
+  if (!(g.mix ? g.P <= 5 : g.wide) || blocks > nsm) return false;
+  double vox = 0.0;
+  for (int ci : g.chains) {
+    const Dataset &d = ctx->ds[ctx->ch[ci].dataset];
+    if (gains_by_release(g, d.N)) vox += (double)d.V;
+  }
+  return vox >= 0.5 * g.vox;
+}
+
+// Which of a lane's outcome words has the wait in its middle: at about three
+// quarters of the subjects, of many a little earlier (blocks come to differ by
+// more: 75,000 voxels, N = 400, P = 4 88 us at 304, 70 at 288).
+int release_word(int N, int lanes, bool mix) {
+  const int at = std::min((int)((int64_t)N * 3 / 4), N / 2 + 75);
+  const int word = at / lanes / 32;
+  return mix && N >= 64 ? std::max(word, 1) : word;
 }
 
 // Threads per block of a group's colour kernels: 256, or 128 where that leaves
@@ -474,25 +521,23 @@ bsg_status build_plan(bsg_ctx *ctx) {
     g.threads = g.fp64 ? kF64Threads
                        : group_threads(g, blocks(kMaxThreads), blocks(kSmallBlock), nsm,
                                        ctx->threads, ctx->threads_set);
-    // A t/logit grid of up to one block per SM with much work per voxel waits
-    // for the kernel before it: started early, beside the blocks of that one,
-    // two of its own can come to share an SM, which costs more than the overlap
-    // gives (38,456 voxels, 151 blocks, N = 1200, P = 3 logistic: 597 us per
-    // sweep early, 506 after).  (Above P = 5 an SM has room for one only.)
-    g.early = !(g.mix && g.P <= 5 && g.threads == kMaxThreads && blocks(kMaxThreads) <= nsm &&
-                g.subj_vox >= 256.0 * g.vox);
     const bool eligible = !g.mix && !g.fp64 && (g.wm_any || (ctx->lpv == 1 && !ctx->tc));
     g.wide = eligible && (ctx->step == 16 ||
                           (ctx->step == 0 && group_wide(g, blocks(g.threads), nsm)));
+    g.release = group_release(ctx, g, blocks(g.threads), nsm);
     // studies with the most subjects first: their blocks take longest, and a
     // launch ends soonest when those do not start last
     std::stable_sort(g.chains.begin(), g.chains.end(), [&](int x, int y) {
       return ctx->ds[ctx->ch[x].dataset].N > ctx->ds[ctx->ch[y].dataset].N;
     });
-    for (int ci : g.chains)
+    for (int ci : g.chains) {
+      const Dataset &d = ctx->ds[ctx->ch[ci].dataset];
+      const int release =
+          g.release && gains_by_release(g, d.N) ? release_word(d.N, lanes, g.mix) : -1;
       for (int c = 0; c < 2; ++c)
-        map_chain(g.map[c], ci, ctx->ch[ci].dataset,
-                  (int)ctx->ds[ctx->ch[ci].dataset].vox[c].size(), g.threads / lanes);
+        map_chain(g.map[c], ci, ctx->ch[ci].dataset, (int)d.vox[c].size(), g.threads / lanes,
+                  release);
+    }
   }
   for (auto &g : ctx->groups) {
     for (int c = 0; c < 2; ++c) {
@@ -523,6 +568,10 @@ cudaError_t launch_colour(bsg_ctx *ctx, const Group &g, int c, cudaStream_t st, 
   if (g.fp64)
     return launch_fp64(g.P, g.fp64, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c,
                        st);
+  if (g.release)
+    return (g.one ? launch_fused_rel_one : launch_fused_rel)(
+        g.P, g.threads, g.mix, g.wm_any, ctx->d_ds, ctx->d_ch, g.d_map[c],
+        (int)g.map[c].size(), c, st, pdl);
   if (g.mix)
     return (g.one ? launch_fused_mix_one : launch_fused_mix)(
         g.P, g.threads, ctx->d_ds, ctx->d_ch, g.d_map[c], (int)g.map[c].size(), c, st, pdl);
@@ -552,7 +601,7 @@ cudaError_t enqueue_group(bsg_ctx *ctx, const Group &g, cudaStream_t st) {
     // predictive pass lies between them (its kernels start their successors
     // only after the wait that completes the colour-1 kernel)
     const bool pdl =
-        ctx->pdl && g.early && !(c == 0 && g.wm_any && g.pred.empty()) && !g.fp64;
+        ctx->pdl && !(c == 0 && g.wm_any && g.pred.empty()) && !g.fp64;
     e = launch_colour(ctx, g, c, st, pdl);
     if (e != cudaSuccess) return e;
   }

@@ -65,8 +65,12 @@ constexpr int fused_min_blocks() {
 // subject pair at P = 5, 43 % of its time) fall by 1 / P; us per sweep with
 // and without, 230,285 voxels: N = 1000 P = 2 439 / 455, P = 5 503 / 516, P =
 // 8 566 / 577; N = 300 P = 3 152 / 158; 24 replicates 274 / 281.
+// REL: the dependency protocol's wait (below) is taken within the subject loop, in
+// the middle of the outcome word that the block map names, for grids of up to
+// one block per SM (group_release); the same arithmetic.  Forms of their own, as
+// the check costs the kernels that do not need it 1 to 2 % (logistic, P = 5, 5 %).
 template <int P, int LPV, bool SUPP, bool MIX = false, bool WMU = false, bool TC = false,
-          bool WIDE = false, bool ONE = false>
+          bool WIDE = false, bool ONE = false, bool REL = false>
 __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
                                   fused_min_blocks<P, MIX, WIDE>())
     fused_colour_kernel(const DatasetDev *__restrict__ dsv,
@@ -86,6 +90,8 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
   constexpr bool PAIRX = !MIX && !SUPP;
   static_assert(!ONE || (!SUPP && !TC && (MIX || LPV == 1) && P > 1),
                 "the intercept form serves the production kernels");
+  static_assert(!REL || (!SUPP && !TC && (MIX || WIDE)),
+                "the early release serves the forms that small grids run");
   constexpr int P0 = ONE ? 1 : 0;  // first staged column
   constexpr int PP = P - P0 <= 4 ? 4 : 8;  // design row padded to float4s
   constexpr int RW = 2 * ((P - P0 + 1) & ~1);  // floats per pair row
@@ -525,6 +531,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           if constexpr (TAB) return philox_qv(pq[c], vlane, key);
           return philox(make_uint4((i00 >> 1) + c, (uint32_t)v, sweep, cid | kTagPhi), key);
         };
+        [[maybe_unused]] const bool release = REL && ((i0 >> 5) + wl) / LPV == bm.release;
         // MIX: the weights phi of a group of four subjects are loaded one
         // group ahead (the stores of the current group may alias as far as
         // the compiler knows, so it would not hoist them itself)
@@ -535,6 +542,12 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           const int nb = TC ? 32 : nbits;
 #pragma unroll 1
           for (int b = 0; b < nb;) {
+            if constexpr (REL) {
+              if (release && b == 16) {
+                cudaGridDependencySynchronize();
+                cudaTriggerProgrammaticLaunchCompletion();
+              }
+            }
             const uint32_t i = i00 + (uint32_t)b;
             auto step = [&](auto gsz, auto rag) {
               constexpr int G = decltype(gsz)::value;
@@ -578,6 +591,12 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
             }
             const uint4 r = zcall(b >> 2);
             if constexpr (MIX) {
+              if constexpr (REL) {
+                if (release && b == 16) {
+                  cudaGridDependencySynchronize();
+                  cudaTriggerProgrammaticLaunchCompletion();
+                }
+              }
               group4_mix(xo + b, yw, r, i, gpair(b >> 1), gpair((b >> 1) + 1), phc);
               yw >>= 4;
             } else {
@@ -594,6 +613,12 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           }
         } else {
           for (int b = 0; b < nbits; b += 4) {
+            if constexpr (REL) {
+              if (release && b == 16) {
+                cudaGridDependencySynchronize();
+                cudaTriggerProgrammaticLaunchCompletion();
+              }
+            }
             const uint32_t i = i00 + (uint32_t)b;
             const uint4 r = zcall(b >> 2);
             const uint4 g0 = gpair(b >> 1), g1 = gpair((b >> 1) + 1);
@@ -685,7 +710,9 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
   // and the outcome bits, all final since this colour's previous launch.
   // The beta update needs Omega and the other colour's new coefficients,
   // written by the previous kernel in the stream: wait for its completion
-  // here, and only then let the next kernel start its own latent phase.
+  // here, and only then let the next kernel start its own latent phase.  (REL:
+  // waited and let in earlier, within the subject loop; the same holds from
+  // there on, and a second wait returns at once.)
   // (Without a programmatic launch both calls return at once.)
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
@@ -1058,7 +1085,7 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
 // block of the previous kernel in the stream has passed its dependency
 // point.
 template <int P, int LPV, bool SUPP, bool MIX = false, bool WMU = false, bool TC = false,
-          bool WIDE = false, bool ONE = false>
+          bool WIDE = false, bool ONE = false, bool REL = false>
 cudaError_t launch_one(int nblocks, int threads, cudaStream_t st, bool pdl,
                        const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
                        int colour, const Supplied &sup) {
@@ -1075,8 +1102,8 @@ cudaError_t launch_one(int nblocks, int threads, cudaStream_t st, bool pdl,
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, fused_colour_kernel<P, LPV, SUPP, MIX, WMU, TC, WIDE, ONE>, ds,
-                            ch, map, colour, sup);
+  return cudaLaunchKernelEx(&cfg, fused_colour_kernel<P, LPV, SUPP, MIX, WMU, TC, WIDE, ONE, REL>,
+                            ds, ch, map, colour, sup);
 }
 
 // The dynamic shared memory opt-in of one tensor-core instantiation.

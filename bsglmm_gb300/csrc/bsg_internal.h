@@ -140,7 +140,8 @@ struct BlockMap {
   int32_t chain;
   int32_t start;    // first colour position (fused) or merged position (post)
   int32_t dataset;  // the chain's (colour kernels: one dependent load less)
-  int32_t pad;
+  int32_t release;  // REL colour kernels: which of a lane's outcome words (0, 1,
+                    // ...) has the dependency protocol's wait in its middle
 };
 
 // ---- launchers (bsg_kernels.cu) ----------------------------------------
@@ -182,6 +183,15 @@ cudaError_t launch_fused_one(int P, int threads, bool wmu, const DatasetDev *ds,
 cudaError_t launch_fused_one_wide(int P, int threads, bool wmu, const DatasetDev *ds,
                                   ChainDev *ch, const BlockMap *map, int nblocks, int colour,
                                   cudaStream_t st, bool pdl);
+// The REL forms (the next kernel let in within the subject loop): the probit and
+// beta_WM 16-subject step and the t/logit links up to P = 5 (bsg_fused_rel.cu,
+// bsg_fused_rel_one.cu; _one: first design column all ones, P > 1).
+cudaError_t launch_fused_rel(int P, int threads, bool mix, bool wmu, const DatasetDev *ds,
+                             ChainDev *ch, const BlockMap *map, int nblocks, int colour,
+                             cudaStream_t st, bool pdl);
+cudaError_t launch_fused_rel_one(int P, int threads, bool mix, bool wmu,
+                                 const DatasetDev *ds, ChainDev *ch, const BlockMap *map,
+                                 int nblocks, int colour, cudaStream_t st, bool pdl);
 // The colour kernel of FP64 chains (bsg_fp64.cu): `lanes` (1 or kF64Lanes)
 // lanes per voxel, blocks of kF64Threads, Philox variates, probit link.
 cudaError_t launch_fp64(int P, int lanes, const DatasetDev *ds, ChainDev *ch,
