@@ -410,7 +410,7 @@ def run_ours(args, rank, world, local):
     ch = s.add_chain(ds, seed=chain_seed(rank), burnin=0, thin=1)
     if args.lpv or args.threads:
         s.set_tuning(args.lpv, args.threads)
-    lpv, thr = s.tuning()
+    lpv, thr = s.tuning()[0], s.block_threads(ch)
     step = s.step_subjects()
     flushbuf = torch.empty(L2_FLUSH_BYTES, dtype=torch.uint8, device=f"cuda:{local}")
 

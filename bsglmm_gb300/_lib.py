@@ -34,6 +34,7 @@ SIGNATURES = {
     "bsg_add_chain": (_i32, [_P, _i32, _P, C.POINTER(_i32)]),
     "bsg_set_tuning": (_i32, [_P, _i32, _i32]),
     "bsg_get_tuning": (_i32, [_P, C.POINTER(_i32), C.POINTER(_i32)]),
+    "bsg_get_block_threads": (_i32, [_P, _i32, C.POINTER(_i32)]),
     "bsg_set_tensor_xz": (_i32, [_P, _i32]),
     "bsg_set_step_subjects": (_i32, [_P, _i32]),
     "bsg_get_step_subjects": (_i32, [_P, C.POINTER(_i32)]),

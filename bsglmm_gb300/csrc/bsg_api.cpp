@@ -1063,11 +1063,12 @@ bsg_status bsg_set_tuning(bsg_ctx *ctx, int32_t lanes_per_voxel,
                           int32_t block_threads) {
   if (!ctx) return BSG_ERR_INVALID;
   const int lpv = lanes_per_voxel ? lanes_per_voxel : ctx->lpv;
-  const int thr = block_threads ? block_threads : ctx->threads;
+  const bool per_group = block_threads == BSG_THREADS_PER_GROUP;
+  const int thr = per_group ? kMaxThreads : block_threads ? block_threads : ctx->threads;
   if (!fused_supported(1, lpv, thr))
     return fail(ctx, BSG_ERR_UNSUPPORTED,
                 "lanes_per_voxel in {1,2,4,8}, block_threads in {64,128,256}");
-  const bool set = ctx->threads_set || block_threads;
+  const bool set = !per_group && (ctx->threads_set || block_threads);
   if (lpv != ctx->lpv || thr != ctx->threads || set != ctx->threads_set) {
     ctx->lpv = lpv;
     ctx->threads = thr;
@@ -1120,6 +1121,17 @@ bsg_status bsg_get_tuning(const bsg_ctx *ctx, int32_t *lpv, int32_t *thr) {
   if (!ctx) return BSG_ERR_INVALID;
   if (lpv) *lpv = ctx->lpv;
   if (thr) *thr = ctx->threads;
+  return BSG_OK;
+}
+
+bsg_status bsg_get_block_threads(bsg_ctx *ctx, int32_t chain, int32_t *block_threads) {
+  if (!valid_chain(ctx, chain) || !block_threads) return BSG_ERR_INVALID;
+  CK(cudaSetDevice(ctx->device));
+  bsg_status s = build_plan(ctx);
+  if (s) return s;
+  for (const auto &g : ctx->groups)
+    if (std::find(g.chains.begin(), g.chains.end(), (int)chain) != g.chains.end())
+      *block_threads = g.threads;
   return BSG_OK;
 }
 
@@ -1747,16 +1759,18 @@ bsg_status bsg_autotune(bsg_ctx *ctx, int32_t sweeps, int32_t *best_lpv,
     bsg_status s = bsg_checkpoint(ctx, (int32_t)i, saved[i].data(), (int64_t)saved[i].size());
     if (s) return s;
   }
-  const int lpvs[] = {1, 2, 4, 8}, thrs[] = {64, 128, 256};
+  // block sizes: one for all groups, or each group's own (the default)
+  const int lpvs[] = {1, 2, 4, 8}, thrs[] = {BSG_THREADS_PER_GROUP, 64, 128, 256};
   double best = 1e300;
-  int bl = ctx->lpv, bt = ctx->threads, bstep = ctx->step;
+  int bl = ctx->lpv, bt = ctx->threads_set ? ctx->threads : BSG_THREADS_PER_GROUP;
+  int bstep = ctx->step;
   bool btc = ctx->tc;
   for (int lpv : lpvs)
     for (int thr : thrs)
       for (int tc = 0; tc < (lpv == 1 ? 2 : 1); ++tc)  // X'Z: SIMT, tensor cores
         for (int step : {0, 16, 8}) {  // subjects per step: per group, 16, 8
           if (step && (lpv != 1 || tc)) continue;  // those take the 8-subject step
-          if (thr / lpv < 8) continue;
+          if (thr > 0 && thr / lpv < 8) continue;
           bsg_status s = bsg_set_tuning(ctx, lpv, thr);
           if (!s) s = bsg_set_tensor_xz(ctx, tc);
           if (!s) s = bsg_set_step_subjects(ctx, step);
@@ -1779,7 +1793,7 @@ bsg_status bsg_autotune(bsg_ctx *ctx, int32_t sweeps, int32_t *best_lpv,
   if (!s) s = bsg_set_step_subjects(ctx, bstep);
   if (s) return s;
   if (best_lpv) *best_lpv = bl;
-  if (best_threads) *best_threads = bt;
+  if (best_threads) *best_threads = ctx->threads;
   return BSG_OK;
 }
 

@@ -98,6 +98,8 @@ class Sampler:
         return out.value
 
     def set_tuning(self, lanes_per_voxel: int = 0, block_threads: int = 0):
+        """Lanes per voxel (1, 2, 4, 8) and threads per block (64, 128, 256;
+        -1: each launch group's own, the default); 0 keeps the current."""
         self._check(self._L.bsg_set_tuning(self._h, lanes_per_voxel,
                                            block_threads), "bsg_set_tuning")
 
@@ -124,6 +126,13 @@ class Sampler:
         self._check(self._L.bsg_get_tuning(self._h, C.byref(a), C.byref(b)),
                     "bsg_get_tuning")
         return a.value, b.value
+
+    def block_threads(self, chain: int = 0) -> int:
+        """Threads per block that the plan runs the chain's kernels in."""
+        n = C.c_int32()
+        self._check(self._L.bsg_get_block_threads(self._h, chain, C.byref(n)),
+                    "bsg_get_block_threads")
+        return n.value
 
     def info(self, dataset: int = 0) -> dict:
         return dict(self._ds[dataset])

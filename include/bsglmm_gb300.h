@@ -88,12 +88,18 @@ bsg_status bsg_add_chain(bsg_ctx *ctx, int32_t dataset_id,
                          const bsg_chain_desc *desc, int32_t *chain_id);
 /* Tile shape of the fused colour kernel: lanes per voxel (1, 2, 4, 8) and
  * threads per block (64, 128, 256); 0 keeps the current choice.  Until a
- * block size is set, each launch group takes 256 or, where that spreads a
- * small grid more evenly over the SMs, 128 (the results are the same). */
+ * block size is set, and again with BSG_THREADS_PER_GROUP, each launch group
+ * takes 256 or, where that spreads a small grid more evenly over the SMs, 128
+ * (the results are the same).  bsg_get_tuning reports 256 then;
+ * bsg_get_block_threads gives the block size that the plan runs a chain in
+ * (FP64 chains have one of their own). */
+#define BSG_THREADS_PER_GROUP (-1)
 bsg_status bsg_set_tuning(bsg_ctx *ctx, int32_t lanes_per_voxel,
                           int32_t block_threads);
 bsg_status bsg_get_tuning(const bsg_ctx *ctx, int32_t *lanes_per_voxel,
                           int32_t *block_threads);
+bsg_status bsg_get_block_threads(bsg_ctx *ctx, int32_t chain,
+                                 int32_t *block_threads);
 
 /* X'(Z - beta_WM WM) of the probit colour kernel (the reference's loop at
  * covarGPU.cu:327-351) on the tensor cores: a BF16x3 split product (x = hi +
@@ -254,12 +260,13 @@ int64_t bsg_checkpoint_size(const bsg_ctx *ctx, int32_t chain);
 bsg_status bsg_checkpoint(bsg_ctx *ctx, int32_t chain, void *buf, int64_t size);
 bsg_status bsg_restore(bsg_ctx *ctx, int32_t chain, const void *buf,
                        int64_t size);
-/* Times each supported tile shape (lanes per voxel x threads per block,
- * and at one lane per voxel both X'Z paths of bsg_set_tensor_xz and, on
- * the SIMT path, the settings 0, 16 and 8 of bsg_set_step_subjects) on the
- * context's chains for `sweeps` sweeps, keeps the fastest (the X'Z path and
- * the step setting stay set on the context) and puts every chain back to
- * its state before the call. */
+/* Times each supported tile shape (lanes per voxel x threads per block, one
+ * size for all launch groups or each group's own, and at one lane per voxel
+ * both X'Z paths of bsg_set_tensor_xz and, on the SIMT path, the settings 0,
+ * 16 and 8 of bsg_set_step_subjects) on the context's chains for `sweeps`
+ * sweeps, keeps the fastest (the X'Z path and the step setting stay set on the
+ * context; lanes_per_voxel and block_threads as bsg_get_tuning gives them) and
+ * puts every chain back to its state before the call. */
 bsg_status bsg_autotune(bsg_ctx *ctx, int32_t sweeps, int32_t *lanes_per_voxel,
                         int32_t *block_threads);
 
