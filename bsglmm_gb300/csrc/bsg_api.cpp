@@ -1087,6 +1087,7 @@ bsg_status bsg_set_tensor_xz(bsg_ctx *ctx, int32_t enable) {
     if (on) CK(prepare_fused_tc());
     clear_graphs(ctx);  // the segments hold the other kernel
     ctx->tc = on;
+    ctx->plan_valid = false;  // so may the groups' choice of the step
   }
   return BSG_OK;
 }

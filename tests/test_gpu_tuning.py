@@ -69,3 +69,25 @@ def test_sizes_per_group_come_back():
                 s.block_threads(2)
     for o in out[1:]:
         assert all(np.array_equal(x, y) for x, y in zip(o, out[0]))
+
+
+@pytest.mark.parametrize("first", [True, False])
+def test_tensor_xz_switch_on_a_running_context(first):
+    """Switched after the plan was built, the tensor-core X'Z is what runs:
+    the same chain as with the plan rebuilt (another block size, same results)."""
+    import bsglmm_gb300 as bsg
+    st = synth.small_study(9, shape=(12, 11, 10), N=70, P=4, S=1)
+    covar = st.covar if first else np.ascontiguousarray(st.covar[::-1])
+    out = []
+    for rebuild in (False, True):
+        with bsg.Sampler() as s:
+            ch = s.add_chain(s.add_dataset(st.mask, covar, st.data, 1), seed=5)
+            s.run(1)
+            assert s.step_subjects() == 16
+            s.set_tensor_xz(True)
+            if rebuild:
+                s.set_tuning(1, 64)
+            s.run(1)
+            assert s.step_subjects() == 8
+            out.append(s.beta(ch))
+    assert np.array_equal(out[0], out[1])
