@@ -1188,8 +1188,8 @@ bsg_status bsg_step_host(bsg_ctx *ctx, int32_t chain, const double *omega_in,
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->pin_busy = false;
   }
-  if (!ctx->pin) {
-    CK(cudaHostAlloc(&ctx->pin, need, cudaHostAllocMapped));
+  if (!ctx->pin_dev) {  // (set last: never staging without its device address)
+    if (!ctx->pin) CK(cudaHostAlloc(&ctx->pin, need, cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer(&ctx->pin_dev, ctx->pin, 0));
   }
   char *base = (char *)ctx->pin, *dev = (char *)ctx->pin_dev;
@@ -1201,10 +1201,14 @@ bsg_status bsg_step_host(bsg_ctx *ctx, int32_t chain, const double *omega_in,
     for (int i = 0; i < P * P; ++i) in_d[i] = omega_in[i];
     CK(launch_stage_in((double *)dev, c.dev.omega_d, c.dev.omega_f, P * P, ctx->stream));
   }
-  // one or two sweeps go kernel by kernel: between the staging kernels a graph
-  // costs more than their launches (20^3 study, one sweep: 52.7 us per step
-  // with it, 48.6 without; four sweeps: 112 either way)
-  if (nsweeps > 2) {
+  // one or two sweeps of one launch group go kernel by kernel: between the staging
+  // kernels a graph costs more than their launches, but not than those of several
+  // groups with the events that join them.  us per step of 20^3 studies, N = 50,
+  // kernel by kernel / as a graph: one group, one sweep 41.7 / 44.3, two 58.2 /
+  // 60.7 (with the predictive pass 68.9 / 69.9, 109.9 / 110.3), three 85.6 / 81.8;
+  // two groups 51.6 / 49.8 and 75.2 / 69.2, three 58.5 / 54.5 and 87.6 / 75.6,
+  // five 75.6 / 64.8 and 117.8 / 95.2.
+  if (nsweeps > 2 || ctx->groups.size() > 1) {
     if ((s = bsg_run(ctx, nsweeps))) return s;
   } else if (nsweeps > 0) {
     CK(enqueue_sweeps(ctx, ctx->stream, nsweeps));
