@@ -266,14 +266,27 @@ std::string status_text(int bits) {
 
 constexpr int kParityThreads = 128;  // tile of the supplied-variate sweep
 
-// Lanes per voxel of an FP64 chain: four while one lane each would put fewer
-// than eight warps on an SM of a GB300 (152 x 8 x 32 voxels of a colour), one
-// above, where four would only idle three lanes of each coefficient draw.
-// By the study alone, so that a chain's sums do not depend on what else its
-// context holds.  Measured at 9,424 voxels a colour, N = 117, P = 4: 0.69 ms
-// per sweep with one lane, 0.44 ms with four.
+// Lanes per voxel of an FP64 chain: four where they shorten its sweeps, else one.
+// Four spread a voxel's subjects over four times the warps, but leave three of
+// four lanes idle in the coefficient draw: with one lane it takes the time of
+// about E = 5 P subjects, with four that of 3.5 E of theirs.  A subject takes
+// `fill` of its one-lane time with four, by how far one lane each fills the FP64
+// pipe: measured 0.2 at 2,400 voxels a colour, 0.45 at 9,600, 0.64 at 12,800 and
+// 0.85 at 18,400 (152 SMs: half a warp, 2, 2.6 and 3.8 warps on each).  By the
+// study alone, so that a chain's sums depend neither on what else its context
+// holds nor on the GPU.  us per sweep, one lane / four, in voxels a colour:
+//    2,400  P = 4, N = 6 118 / 111, N = 40 290 / 152
+//    9,600  P = 2, N = 12 113 / 114, N = 20 151 / 149; P = 4, N = 20 194 / 215, N =
+//           30 243 / 214; P = 8, N = 40 424 / 436, N = 60 542 / 477
+//   12,800  P = 2, N = 30 209 / 204; P = 4, N = 30 257 / 295, N = 117 721 / 631;
+//           P = 8, N = 117 920 / 1090, N = 400 2638 / 2425
+//   18,400  P = 2, N = 117 647 / 691, N = 400 2054 / 1891; P = 4, N = 6 130 / 316,
+//           N = 200 1156 / 1215, N = 400 2214 / 2114
+//   32,000  P = 2, N = 6 134 / 361, N = 400 3594 / 3677
 int f64_lanes(const Dataset &d) {
-  return std::max(d.vox[0].size(), d.vox[1].size()) < 38912 ? kF64Lanes : 1;
+  const double n = (double)std::max(d.vox[0].size(), d.vox[1].size());
+  const double fill = std::min(0.88, n / 20500.0), E = 5.0 * d.P;
+  return n < 20000 && fill * (d.N + 3.5 * E) < d.N + E ? kF64Lanes : 1;
 }
 
 // Whether a chain runs the kernels for a first design column of ones.
