@@ -14,6 +14,7 @@
 // operations: about 55 + 2 P per subject and voxel.  CUDA's normcdf and
 // normcdfinv, which it used before, took some 330 and 2,120 instructions in
 // all, since the lanes of a warp go down both branches of each.
+#include "../../include/bsglmm_gb300.h"
 #include "bsg_mills_table.h"
 #include "bsg_wishart.cuh"
 
@@ -456,6 +457,41 @@ __global__ void __launch_bounds__(kF64Threads)
   if (warp == 1) sweep_end_warp(ch, d, tot, sweep_ll, kept, 0, lane);
 }
 
+// Self-check of the latent draw: t[i] = tn_lower_inv_d(a[i], k[i]).
+__global__ void draw64_selftest_kernel(int64_t n, const double *a, const uint32_t *k,
+                                       double *t) {
+  __shared__ DrawTables tb;
+  load_tables(tb, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) t[i] = tn_lower_inv_d(a[i], k[i], tb);
+}
+
+// Self-check of div_by against the division, bit for bit, over mantissas of all kinds
+// and exponents within 2^40, and of rsqrt_step: its largest relative error, in
+// units of 2^-53, from the remainder 1 - d y^2 taken to twice the precision.
+__global__ void quotient_selftest_kernel(int64_t n, uint32_t k0, uint32_t k1,
+                                         unsigned long long *out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint4 r = philox1(make_uint4((uint32_t)i, (uint32_t)(i >> 32), 2u, 0xA5u), k0, k1);
+  auto mant = [](uint32_t w, int kind) -> uint32_t {  // random, or next to a power of two
+    const uint32_t m = w & 0x7fffffu;
+    return kind == 0 ? m & 7u : kind == 1 ? 0x7fffffu - (m & 7u) : m;
+  };
+  auto expo = [](uint32_t w) -> uint32_t { return 127u - 40u + (w >> 24) % 81u; };
+  const float x = __uint_as_float((r.x & 0x80000000u) | expo(r.y << 1) << 23 |
+                                  mant(r.x, (int)(r.z & 7u)));
+  const float g = __uint_as_float(expo(r.y >> 9 << 24 | r.y) << 23 |
+                                  mant(r.y, (int)(r.z >> 3 & 7u)));
+  if (__float_as_uint(div_by(x, g, 1.f / g)) != __float_as_uint(x / g)) atomicAdd(out, 1ull);
+  const double d = __hiloint2double((int)((1023u - 60u + (r.z >> 8) % 121u) << 20 |
+                                          (r.w & 0xfffffu)), (int)(r.x * 2654435761u ^ r.w));
+  const double y = rsqrt_step(d), y2 = y * y, lo = fma(y, y, -y2);
+  const double e = 0.5 * (fma(-d, y2, 1.0) - d * lo);
+  atomicMax(out + 1, (unsigned long long)(fabs(e) * 0x1p53 * 1000.0));
+}
+
 }  // namespace
 
 cudaError_t launch_fp64(int P, int lanes, const DatasetDev *ds, ChainDev *ch,
@@ -486,3 +522,45 @@ cudaError_t launch_fp64(int P, int lanes, const DatasetDev *ds, ChainDev *ch,
 }
 
 }  // namespace bsg
+
+extern "C" bsg_status bsg_selftest_draw64(int32_t device, int64_t n, const double *a,
+                                          const uint32_t *k, double *t) {
+  if (n < 1 || n > (1 << 26) || !a || !k || !t) return BSG_ERR_INVALID;
+  int nd = 0;
+  if (cudaGetDeviceCount(&nd) != cudaSuccess || nd == 0) return BSG_ERR_NO_DEVICE;
+  if (cudaSetDevice(device) != cudaSuccess) return BSG_ERR_INVALID;
+  double *buf = nullptr;  // a, t, k
+  if (cudaMalloc(&buf, (size_t)n * 20) != cudaSuccess) return BSG_ERR_CUDA;
+  uint32_t *dk = (uint32_t *)(buf + 2 * n);
+  cudaError_t e = cudaMemcpy(buf, a, (size_t)n * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dk, k, (size_t)n * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    bsg::draw64_selftest_kernel<<<(unsigned)((n + 127) / 128), 128>>>(n, buf, dk, buf + n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(t, buf + n, (size_t)n * 8, cudaMemcpyDeviceToHost);
+  cudaFree(buf);
+  return e == cudaSuccess ? BSG_OK : BSG_ERR_CUDA;
+}
+
+extern "C" bsg_status bsg_selftest_quotients(int32_t device, int64_t n, uint64_t seed,
+                                             int64_t *mismatches, double *rsqrt_error) {
+  if (n < 1 || n > (1ll << 36) || !mismatches || !rsqrt_error) return BSG_ERR_INVALID;
+  int nd = 0;
+  if (cudaGetDeviceCount(&nd) != cudaSuccess || nd == 0) return BSG_ERR_NO_DEVICE;
+  if (cudaSetDevice(device) != cudaSuccess) return BSG_ERR_INVALID;
+  unsigned long long *out = nullptr, h[2] = {0, 0};
+  if (cudaMalloc(&out, sizeof(h)) != cudaSuccess) return BSG_ERR_CUDA;
+  cudaError_t e = cudaMemset(out, 0, sizeof(h));
+  if (e == cudaSuccess) {
+    bsg::quotient_selftest_kernel<<<(unsigned)((n + 255) / 256), 256>>>(
+        n, (uint32_t)seed, (uint32_t)(seed >> 32), out);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(h, out, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(out);
+  if (e != cudaSuccess) return BSG_ERR_CUDA;
+  *mismatches = (int64_t)h[0];
+  *rsqrt_error = (double)h[1] / 1000.0;
+  return BSG_OK;
+}

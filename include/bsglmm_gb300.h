@@ -334,6 +334,17 @@ bsg_status bsg_fp32_peak(int32_t device, double *tflops);
  * two forms agree).  No counterpart in the reference. */
 bsg_status bsg_selftest_pairs(int32_t device, int64_t n, uint64_t seed,
                               int64_t *mismatches);
+/* The FP64 chain's latent draw by itself: t[i] = the draw of N(0, 1) on (a[i],
+ * inf) by inversion of u = (k[i] + 1/2) 2^-32, for -37 < a[i] <= 5 (host
+ * arrays of n, at most 2^26). */
+bsg_status bsg_selftest_draw64(int32_t device, int64_t n, const double *a,
+                               const uint32_t *k, double *t);
+/* Self-check on n seeded random inputs of the triangular solves' quotients by
+ * reciprocal against the division, bit for bit (*mismatches), and of the Omega
+ * draw's reciprocal square root (*rsqrt_error: the largest relative error, in
+ * units of 2^-53). */
+bsg_status bsg_selftest_quotients(int32_t device, int64_t n, uint64_t seed,
+                                  int64_t *mismatches, double *rsqrt_error);
 
 #ifdef __cplusplus
 }
