@@ -45,7 +45,7 @@ struct Chain {
 struct Group {
   int P = 0;
   bool mix = false;     // t/logit chains (scale-mixture colour kernel)
-  bool wm_any = false;  // its chains draw beta_WM: colour 0 waits for it
+  bool wm_any = false;  // its chains draw beta_WM, which colour 0 needs from its start
   int fp64 = 0;         // lanes per voxel of FP64 chains (fp64_colour_kernel,
                         // no early start); 0: FP32
   bool wide = false;    // the 16-subject whole-word step (bsg_fused_wide.cu)

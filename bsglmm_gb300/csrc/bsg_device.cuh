@@ -80,12 +80,13 @@ __device__ __forceinline__ uint4 philox1(uint4 c, uint32_t a, uint32_t b) {
 }
 
 // Philox over one thread's counters (q, v, sweep, w3), where only v differs
-// between the threads of a block and only q between a thread's calls.  Until
-// round 3 every product and xor of the ten rounds depends on q alone or on v
-// alone: philox_q gives the four words that depend on q (one thread per q,
-// kept in shared memory for the block), PhiloxLane the two that depend on v
-// (registers), and philox_qv finishes from both: the same words as philox()
-// with 15 of its 20 wide products and 17 of its 20 xors.
+// between the threads of a block and only q between a thread's calls.  In the
+// generator's first rounds, up to the middle of its third, every product and
+// xor depends on q alone or on v alone: philox_q gives the four words that
+// depend on q (one thread per q, kept in shared memory for the block),
+// PhiloxLane the two that depend on v (registers), and philox_qv finishes from
+// both: the same words as philox() with 15 of its 20 wide products and 17 of its
+// 20 xors.
 __device__ __forceinline__ uint4 philox_q(uint32_t q, uint32_t sweep, uint32_t w3,
                                           const PhiloxKey &k) {
   const uint32_t z1 = __umulhi(0xD2511F53u, q) ^ w3 ^ k.r1(0), w1 = 0xD2511F53u * q;

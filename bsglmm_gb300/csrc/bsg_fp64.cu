@@ -6,14 +6,14 @@
 // covar.cpp:121-325 and mcmc.cpp:584-651 on the same counters), fast enough
 // to run the long reference chains that the FP32 sampler's maps are
 // measured against at the brain-sized studies, where the CPU would take
-// days.  One thread per voxel, subjects in order, or (studies with too few
-// voxels to fill the GPU) four lanes per voxel.
+// days.  One thread per voxel, subjects in order, or (few voxels, many
+// subjects) four lanes per voxel.
 //
 // What bounds it is the FP64 pipe (two lanes per clock and SM: a warp's
 // operation takes 16 cycles), so the latent draw is written for FP64
-// operations: about 55 + 2 P per subject and voxel.  CUDA's normcdf and
-// normcdfinv, which it used before, took some 330 and 2,120 instructions in
-// all, since the lanes of a warp go down both branches of each.
+// operations: about 55 + 2 P per subject and voxel.  With CUDA's normcdf and
+// normcdfinv, which it used before, an update took some 330 of them, 2,120
+// instructions in all, since the lanes of a warp go down both branches of each.
 #include "../../include/bsglmm_gb300.h"
 #include "bsg_mills_table.h"
 #include "bsg_wishart.cuh"

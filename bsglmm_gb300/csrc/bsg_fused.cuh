@@ -3,9 +3,10 @@
 // subjects from the packed outcome bits, accumulates X'(Z - b_WM WM) in
 // registers (Z never reaches memory), forms the conditional precision
 // Q = X'X + n_v Omega and mean vector, factors Q (once per block for each
-// n_v; per voxel for the t/logit links) and draws beta_v.  With the new beta_v it also adds the kept sweep's FP64 running
-// sums and the column sums, and (colour 1) the voxel's Omega pair products;
-// the last colour-1 block of a chain draws Omega.  A sweep is two launches.
+// n_v; per voxel for the t/logit links) and draws beta_v.  With the new beta_v
+// it also adds the kept sweep's FP64 running sums and the column sums, and
+// (colour 1) the voxel's Omega pair products; the last colour-1 block of a
+// chain draws Omega.  A sweep is two launches.
 //
 // Replaces Z_GPU1 (covarGPU.cu:1368-1428) + Spat_Coef_Probit
 // (covarGPU.cu:293-396) and the CPU updateZ / Spat_Coefff
@@ -138,8 +139,9 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
     sc = d.nb[colour][j];
     v = d.vidx[colour][j];
     wmv = d.wm ? d.wm[v] : 1.f;
-    // beta_WM is final since the previous colour-1 launch: with its update
-    // on, colour-0 launches do not start early (no programmatic launch)
+    // beta_WM is final since the previous colour-1 launch: with its update on,
+    // a colour-0 launch starts early only behind the predictive pass, whose
+    // kernels let it in once the colour-1 kernel is complete
     bwm = *ch.wm_beta * wmv;
 #pragma unroll
     for (int p = 0; p < P; ++p) beta[p] = ch.beta[(size_t)p * Vp + sc];
@@ -532,9 +534,6 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
           return philox(make_uint4((i00 >> 1) + c, (uint32_t)v, sweep, cid | kTagPhi), key);
         };
         [[maybe_unused]] const bool release = REL && ((i0 >> 5) + wl) / LPV == bm.release;
-        // MIX: the weights phi of a group of four subjects are loaded one
-        // group ahead (the stores of the current group may alias as far as
-        // the compiler knows, so it would not hoist them itself)
         if constexpr (PAIRX) {
           // whole steps of kGroups calls, then (the end of a ragged last
           // word) steps of two calls or one, the last one perhaps reaching
@@ -577,6 +576,9 @@ __global__ void __launch_bounds__(MIX && WIDE ? kSmallBlock : kMaxThreads,
             }
           }
         } else if (nbits == 32) {
+          // MIX: the weights phi of a group of four subjects are loaded one
+          // group ahead (the stores of the current group may alias as far as
+          // the compiler knows, so it would not hoist them itself)
           float phc[4] = {1.f, 1.f, 1.f, 1.f}, phx[4] = {1.f, 1.f, 1.f, 1.f};
           if (MIX) {
 #pragma unroll

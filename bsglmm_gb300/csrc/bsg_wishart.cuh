@@ -41,7 +41,8 @@ static __device__ double gamma_mt(double a, uint32_t slot, uint32_t sweep,
 // draws sqrt(chi^2(df - i)) into wd[i], lane q < P(P-1)/2 the normal of
 // the q-th strictly lower entry (row-major) into wd[kMaxP + q].  Run off the
 // Omega draw's dependency chain: by a warp of colour 1 before its wait (FP64
-// chains: by the last colour-0 block).  Returns the lane's error bits.  F64: normals in FP64 (the FP64 chain).
+// chains: by the last colour-0 block).  Returns the lane's error bits.  F64:
+// normals in FP64 (the FP64 chain).
 template <bool F64 = false>
 static __device__ int wishart_draws(const ChainDev &ch, const DatasetDev &d,
                                     long long sweep, int lane, double *wd) {
